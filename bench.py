@@ -171,7 +171,7 @@ def measured_hbm_peak():
 def kernel_source_hash():
     """Hash of the stage kernel's sources (the kernel header and its sector tables)."""
     h = hashlib.sha256()
-    for rel in ("dm-heom_b200/csrc/heom_kernels.cuh", "dm-heom_b200/csrc/pair_tables.inc"):
+    for rel in ("dm-heom_b200/csrc/heom_kernels.cuh", "dm-heom_b200/csrc/row_tables.inc"):
         with open(os.path.join(ROOT, rel), "rb") as f:
             h.update(f.read())
     return h.hexdigest()[:16]

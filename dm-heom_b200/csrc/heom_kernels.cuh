@@ -43,6 +43,7 @@
 namespace heomk {
 
 constexpr int kCtaWarps = 8;
+constexpr int kRowWarps = 4; // warps of a CTA of the N <= 8 stage kernel
 
 __host__ __device__ constexpr int pairs_of(int n) { return n * (n - 1) / 2 + (n + 1) / 2; }
 __host__ __device__ constexpr int team_warps(int n) { return (pairs_of(n) + 31) / 32; }
@@ -81,14 +82,15 @@ struct PairParams {
     const double2* y;                // AXPY against y instead of in (may alias out)
     double2* out;
     double2* acc;                    // accumulate mode
-    double2 alpha;                   // out = alpha * x + beta * L
-    double2 beta;
+    double2 beta;                    // out = (use_x ? x : 0) + beta * L
     double2 acc_beta;                // acc = (acc_init ? in : acc) + acc_beta * L
+    int use_x;
     int acc_init;
     int use_acc;
-    const int32_t* __restrict__ nbr; // [nodes][NW]: (plus, minus) of every slot, padded to NW (multiple of 4)
-    const uint8_t* __restrict__ tup; // [nodes][TWB] tuple bytes, padded to TWB (multiple of 16)
-    const double2* __restrict__ pss; // [nodes]
+    int no_same;                     // leave out pf_same_sum (flow tracking)
+    // one record of rec_bytes(NW, TWB) per ADO: (plus, minus) of every slot as int32, padded to NW (multiple of 4);
+    // the tuple bytes, padded to TWB (multiple of 16); pf_same_sum (double2)
+    const unsigned char* __restrict__ rec;
     const double* __restrict__ hfrag;  // [n_inst][frag_doubles(N)] MMA operand fragments of H / hbar
     const int32_t* __restrict__ inst;  // [nodes] instance of each ADO; NULL when the handle holds one instance
     const double2* __restrict__ gamma0;// [N*N]
@@ -99,14 +101,18 @@ struct PairParams {
 
 enum HKind : int { H_REAL_SYM = 0, H_GENERIC = 1 };
 
+__host__ __device__ constexpr int rec_bytes(int NW, int TWB) { return NW * 4 + TWB + 16; }
+
 // MMA operand fragments of H / hbar, per instance: N <= 8 one 8 x 8 block and
 // two k-slices, N = 9..16 a zero-padded 16 x 16 grid of 2 x 2 blocks and four
 // k-slices.  Layout [kind][block b][k-slice s][lane], lane l = 4g + t:
-// kind 0/1 = Re/Im of hb = H(4s+t, 8b+g) (B operand of w H for block column b),
-// kind 2/3 = Re/Im of ha = -H(8b+g, 4s+t) (A operand of -H w for block row b).
+// kind 0/1 = Re/Im of hb = H(c, 8b+g) (B operand of w H for block column b),
+// kind 2/3 = Re/Im of ha = -H(8b+g, c) (A operand of -H w for block row b), c = frag_col(n, s, t).
 __host__ __device__ constexpr int frag_blocks(int n) { return n <= 8 ? 1 : 2; }
 __host__ __device__ constexpr int frag_slices(int n) { return n <= 8 ? 2 : 4; }
 __host__ __device__ constexpr int frag_doubles(int n) { return 4 * frag_blocks(n) * frag_slices(n) * 32; }
+// column (contraction index) of k-slice s in lane position t: N <= 8 the lane's own columns 2t, 2t+1
+__host__ __device__ constexpr int frag_col(int n, int s, int t) { return n <= 8 ? 2 * t + s : 4 * s + t; }
 __host__ __device__ constexpr int frag_index(int n, int kind, int b, int s, int lane)
 {
     return ((kind * frag_blocks(n) + b) * frag_slices(n) + s) * 32 + lane;
@@ -193,26 +199,64 @@ __device__ __forceinline__ void cmac(double2& acc, const double2 a, const double
 __device__ __forceinline__ double2 ldg2(const double2* p) { return __ldg(p); }
 
 // ---------------------------------------------------------------------------
-// N <= 8: one warp per ADO, commutator on the FP64 tensor pipe.
+// N <= 8: one warp per ADO, one lane per (state, column pair).
 //
-// The tile is zero-padded to 8 x 8.  For k-slice s in {0, 1} lane l = 4r + t
-// needs the MMA operands A = w(r, 4s+t) (for w H) and B = w(4s+t, r) (for
-// H w): the two halves of one pair sector, read from the staged tile.  Eight
-// m8n8k4 MMAs (real H; sixteen for complex H) give C = w H - H w at
-// (r, 2t), (r, 2t+1); the result goes through a swizzled row-major tile to the
-// lane that owns the sector.  The sector order (pair_tables.inc) makes both
-// the operand reads and the exchange reads free of bank conflicts.
+// Lane 4r + t works for state r and the columns 2t, 2t+1 (the tile is
+// zero-padded to 8 x 8): it holds the sectors of the pairs {r, 2t} and
+// {r, 2t+1} (for t = r / 2 the diagonal sector stands for {r, r}).
+//   * Commutator on the FP64 tensor pipe: the row elements (r, 2t+s) are the A
+//     fragment of w H and the column elements (2t+s, r) the B fragment of H w
+//     for k-slice s (k = 2t + s), and the C fragment is (r, 2t), (r, 2t+1):
+//     the lane's own row elements.  Eight m8n8k4 MMAs for real H, sixteen for
+//     complex H.
+//   * Bath terms: the lane reads its two sectors of the neighbours along the
+//     baths of state r only, so the slot's index, sqrt(n) and coefficients are
+//     looked up once for four elements.  They give the row-r terms of the row
+//     elements and the column-r terms of the column elements.
+//   * A sector {r, c} is held by a lane of row r and a lane of row c.  One of
+//     them owns it (row_owned); the other hands over its terms by eight
+//     shuffles, and the owner writes the 32-byte sector.  A sector's first
+//     half is the owner's row element, so that all coefficients are in place.
 //
-// Pipeline: per warp two slots, each filled by 1-D TMA bulk copies (tile,
-// neighbour row, tuple row, pf_same_sum) that complete on the slot's
-// mbarrier; the copies of ADO k+1 fly while ADO k is computed.  Every wait is
-// bounded; on expiry the kernel sets *p.err and the warp stops.
+// Pipeline: per warp two slots, each filled by two 1-D TMA bulk copies (tile,
+// record) that complete on the slot's mbarrier; the copies of ADO k+1 fly
+// while ADO k is computed.  Every wait is bounded; on expiry the kernel sets
+// *p.err and the warp stops.
+//
+// What bounds it: the L1 data pipe (8 states, two slots: 143 wavefronts of 194
+// cycles per ADO and SM; 88 of them shared memory) and the latency of 20 warps
+// per SM.  Measured against a lane per sector, which looked up both sites'
+// slots for two elements (us per stage, one B200): 8 states, two slots, 735,471
+// ADOs 791 -> 547, 74,613 ADOs 76.0 -> 51.8; one slot, 24,310 ADOs 21.5 -> 15.9,
+// 319,770 ADOs 235 -> 200; 7 states, one slot, 6435 ADOs 9.75 -> 6.7; 330 ADOs
+// 4.6 -> 3.1 (mostly the dependent launch).  503 -> 347 instructions and 204 ->
+// 143 wavefronts per ADO; 47 of the 61 fewer are shared memory's, the rest a
+// store that is linear in the lanes (22 -> 8) and owned sectors side by side.
+// A lane table read from the parameter bank has to be held (opaque): reloaded
+// under register pressure it cost 180 instructions per ADO and half the speed.
+// Two slots: the K neighbours are read one ADO ahead and the coefficients come
+// from shared memory (in registers they spill: 1137 us); one slot: the other
+// way round (15.4 against 16.0 us; 16.9 with both ahead).
 // ---------------------------------------------------------------------------
 
+// which of its two sectors lane (r, t) owns: 0 = {r, 2t}, 1 = {r, 2t+1}
+__host__ __device__ constexpr int row_owned(int r, int t)
+{
+    return t == (r >> 1) ? 0 : (r & 1) ^ ((r >> 1) > t ? 1 : 0);
+}
+
+// sector position of pair {r, 2t+s} for lane 4r + t (-1: outside N x N)
+struct RowTab {
+    signed char pos[32][2];
+};
+
+// lane tables of the lockstep kernel: the operand sectors of every lane and
+// which half holds the row element
 struct LaneTab {
-    signed char e1[32], e2[32]; // owned sector: element indices (row-major)
+    signed char e1[32], e2[32]; // sector of lane p: element indices (row-major)
+    signed char ord[32];        // the sectors in the order in which the warps take them
     signed char fs[32][2];      // operand sector of k-slice s (-1: zero padding)
-    signed char ha[32][2];      // half of that sector holding A = w(r, 4s+t)
+    signed char ha[32][2];      // half of that sector holding A = w(r, 2t+s)
 };
 
 // Factored bath coefficients: cplus(n) = chat * sqrt(n+1), kappa(n) = khat * sqrt(n)
@@ -228,7 +272,7 @@ struct CoefTabs {
 
 struct DmmaParams {
     PairParams p;
-    LaneTab lt;
+    RowTab rt; // N <= 8
     CoefTabs ct;
     int* err;
 };
@@ -320,268 +364,364 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity)
 
 __device__ __forceinline__ int swz(int r) { return ((r & 1) << 2) | (r & 1) | (((r >> 1) & 1) << 1); }
 
-// bytes of one pipeline slot and of a warp's shared area for the DMMA kernel
+// bytes of one pipeline slot and of a warp's shared area for the DMMA kernel:
+// the tile, the ADO's record and 16 bytes of zeros (operands outside N x N)
 __host__ __device__ inline int dmma_slot_bytes(int P, int NW, int TWB)
 {
-    return P * 32 + ((NW * 4 + 15) & ~15) + ((TWB + 15) & ~15) + 16;
+    return P * 32 + ((rec_bytes(NW, TWB) + 15) & ~15) + 16;
 }
 __host__ __device__ inline int dmma_warp_bytes(int P, int NW, int TWB)
 {
-    return 2 * dmma_slot_bytes(P, NW, TWB) + 64 * 16 /* exchange tile */ + 16 /* 2 mbarriers */;
+    return 2 * dmma_slot_bytes(P, NW, TWB) + 16 /* 2 mbarriers */;
 }
 __host__ inline size_t dmma_smem_bytes(int P, int W, int NW, int TWB, int LS)
 {
-    return (size_t)dmma_lut_bytes(W, LS) + (size_t)kCtaWarps * dmma_warp_bytes(P, NW, TWB);
+    return (size_t)dmma_lut_bytes(W, LS) + 2 * 32 * 16 + (size_t)kRowWarps * dmma_warp_bytes(P, NW, TWB);
 }
+
+// 32 bytes at src when v >= 0; otherwise a and b keep what they hold
+__device__ __forceinline__ void ld256_if(int v, const double2* src, double2& a, double2& b)
+{
+    asm volatile("{\n .reg .pred q;\n setp.ge.s32 q, %5, 0;\n @q ld.global.v4.f64 {%0,%1,%2,%3}, [%4];\n}\n"
+                 : "+d"(a.x), "+d"(a.y), "+d"(b.x), "+d"(b.y)
+                 : "l"(src), "r"(v));
+}
+
+__device__ __forceinline__ double2 shfl2(double2 v, int src)
+{
+    return make_double2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
+}
+__device__ __forceinline__ double2 sel2(bool q, double2 a, double2 b)
+{
+    return make_double2(q ? a.x : b.x, q ? a.y : b.y);
+}
+
+// a value the compiler has to keep: under register pressure it otherwise loads a lane's table entry from the
+// parameter bank again and again, and a constant load with 32 different addresses takes 32 turns
+__device__ __forceinline__ int opaque(int v)
+{
+    asm volatile("" : "+r"(v));
+    return v;
+}
+
+// dependent launch: the next kernel of the stream may start its prologue; wait
+// until the kernels before this one are complete and their writes visible
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+
+// CTAs of four warps per SM: five (96 registers a thread, 20 warps) where that does not spill (8 states, two
+// slots, 735,471 ADOs: 547 us a stage, against 608 at 16 warps and 789 at 24 with 56 bytes spilled)
+constexpr int row_blocks(int hk, int slt, bool mi) { return hk == H_REAL_SYM && slt <= 2 && !mi ? 5 : 4; }
 
 // MI: the handle holds several instances (p.inst set); each ADO's instance
 // selects its H fragments, reloaded whenever the instance changes.
 // ADJ: apply the adjoint operator L^H instead of L.  The caller passes the
-// tables of -H^H (fragments), conj(pf_same_sum) and conj(gamma0); in the bath
-// terms the roles of the neighbours swap: the plus neighbour enters with
-// conj(khat) sqrt(n+1), the minus neighbour with -/+ i chat sqrt(n).
-template <int N, int HK, int SLT, bool MI, bool ADJ>
-__global__ void __launch_bounds__(kCtaWarps * 32, 2) heom_dmma_stage(const DmmaParams dp)
+// tables of -H^H (fragments) and conj(gamma0); pf_same_sum is conjugated here.
+// In the bath terms the roles of the neighbours swap: the plus neighbour enters
+// with conj(khat) sqrt(n+1), the minus neighbour with -/+ i chat sqrt(n).
+// "K" is the neighbour with the complex coefficient (minus for L, plus for
+// L^H), "C" the one with the imaginary coefficient.
+// GEN: every write mode; otherwise out = in + beta L only (the product form).
+template <int N, int HK, int SLT, bool MI, bool ADJ, bool GEN>
+__global__ void __launch_bounds__(kRowWarps * 32, row_blocks(HK, SLT, MI)) heom_dmma_stage(const __grid_constant__ DmmaParams dp)
 {
     static_assert(N <= 8, "DMMA stage handles N <= 8");
     constexpr int P = pairs_of(N);
+    constexpr bool AHEAD = SLT > 1;            // read the K neighbours one ADO ahead
+    constexpr bool XLATE = SLT > 1;            // read the sector's own values again at the end
+    constexpr bool KREG = SLT == 1;            // coefficients in registers (two slots: they would spill)
+    constexpr int QB = SLT < 2 ? SLT : 2;      // slots whose neighbours are read in one batch
+    constexpr bool ODD = (N & 1) != 0;         // some lanes hold one sector only
+    constexpr unsigned tile_b = P * 32;
     const PairParams& p = dp.p;
     extern __shared__ __align__(128) unsigned char smem[];
     const int W = p.W, LS = p.LS, SL = p.SL;
 
-    double2* s_kh = reinterpret_cast<double2*>(smem);            // 3 * W
+    grid_launch_dependents();
+    double2* s_kh = reinterpret_cast<double2*>(smem);            // [3][W]: kappa_i, kappa_j, kappa_i + kappa_j
     double2* s_sq = s_kh + 3 * W;                                 // LS + 1: (sqrt(n), sqrt(n+1))
     double* s_ch = reinterpret_cast<double*>(s_sq + LS + 1);      // W
     for (int q = threadIdx.x; q < 3 * W; q += blockDim.x) s_kh[q] = dp.ct.khat[q];
     for (int q = threadIdx.x; q < W; q += blockDim.x) s_ch[q] = dp.ct.chat[q];
     for (int q = threadIdx.x; q <= LS; q += blockDim.x)
         s_sq[q] = make_double2(dp.ct.sq[q], q < LS ? dp.ct.sq[q + 1] : 0.0);
-    const int lut = dmma_lut_bytes(W, LS);
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const int slot_b = dmma_slot_bytes(P, p.NW, p.TWB);
-    unsigned char* wbase = smem + lut + warp * dmma_warp_bytes(P, p.NW, p.TWB);
-    double2* xch = reinterpret_cast<double2*>(wbase + 2 * slot_b);      // 8 x 8 swizzled
-    uint64_t* bars = reinterpret_cast<uint64_t*>(wbase + 2 * slot_b + 64 * 16);
-    const int tile_b = P * 32;
-    const int nbr_off = tile_b;
-    const int tup_off = nbr_off + ((p.NW * 4 + 15) & ~15);
-    const int pss_off = tup_off + ((p.TWB + 15) & ~15);
-    const unsigned tx_bytes = (unsigned)(tile_b + p.NW * 4 + p.TWB + 16);
+    const unsigned recb = rec_bytes(p.NW, p.TWB);
+    // per warp: the two mbarriers, then the two slots (tile, record, zeros)
+    double2* s_g0 = reinterpret_cast<double2*>(smem + dmma_lut_bytes(W, LS));
+    unsigned char* wbase = smem + dmma_lut_bytes(W, LS) + 1024 + warp * dmma_warp_bytes(P, p.NW, p.TWB);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(wbase);
+    unsigned char* slot = wbase + 16;           // slot of the current ADO
+    unsigned char* slot_n = slot + slot_b;      // slot of the next one
+    const int tup_off = tile_b + p.NW * 4;
+    const int pss_off = tup_off + p.TWB;
 
-    // lane tables
-    const bool owner = lane < P;
-    const int e1 = owner ? dp.lt.e1[lane] : 0, e2 = owner ? dp.lt.e2[lane] : 0;
-    const int i1 = e1 / N, j1 = e1 - i1 * N, i2 = e2 / N, j2 = e2 - i2 * N;
-    const int diag = (i1 == j1);
-    const int si = i1, sj = j1; // sites of the element pair (diagonal: the two diagonal sites are i1 and i2)
-    const int fs0 = dp.lt.fs[lane][0], fs1 = dp.lt.fs[lane][1];
-    const int ha0 = dp.lt.ha[lane][0], ha1 = dp.lt.ha[lane][1];
+    // ---- this lane's place ----
     const int r = lane >> 2, t = lane & 3;
-    const int xr1 = 8 * i1 + (j1 ^ swz(i1)), xr2 = 8 * i2 + (j2 ^ swz(i2));
-    const int xw0 = 8 * r + ((2 * t) ^ swz(r)), xw1 = 8 * r + ((2 * t + 1) ^ swz(r));
+    const bool odd = row_owned(r, t) != 0;              // owns {r, 2t+1}
+    const bool dga = t == (r >> 1) && !(r & 1);         // its sector 0 is the diagonal one (owned)
+    const bool dgb = t == (r >> 1) && (r & 1);          // its sector 1 is the diagonal one (handed over)
+    const int ps0 = opaque(dp.rt.pos[lane][0]), ps1 = opaque(dp.rt.pos[lane][1]);
+    const int pso = odd ? ps1 : ps0, psg = odd ? ps0 : ps1; // owned, handed over
+    const bool owner = pso >= 0, holds = psg >= 0;
+    // the lane that hands over this lane's owned sector
+    const int giver = t == (r >> 1) ? lane ^ 4 : 4 * (2 * t + (odd ? 1 : 0)) + (r >> 1);
+    // operand offsets in a slot (bytes): row and column element of both sectors
+    const int zero_off = slot_b - 16;
+    const int ro0 = ps0 >= 0 ? ps0 * 32 + (odd ? 16 : 0) : zero_off;
+    const int co0 = ps0 >= 0 ? ps0 * 32 + (odd ? 0 : 16) : zero_off; // diagonal: the second diagonal element
+    const int ro1 = ps1 >= 0 ? ps1 * 32 + (odd ? 0 : 16) : zero_off;
+    const int co1 = ps1 >= 0 ? (dgb ? ro1 : ps1 * 32 + (odd ? 16 : 0)) : zero_off;
+    // negative: no such sector; no C term on it (diagonal)
+    const int no_o = owner ? 0 : -1, no_g = holds ? 0 : -1;
+    const int no_co = dga ? -1 : no_o, no_cg = dgb ? -1 : no_g;
+    const double2* in_o = p.in + 2 * (owner ? pso : 0);
+    const double2* in_g = p.in + 2 * (holds ? psg : 0);
 
-    // operand fragments of H / hbar for k-slice s (zero outside the N x N block):
-    //   hb = H(4s+t, r) (B operand of w H), ha = -H(r, 4s+t) (A operand of -H w);
-    // packed per instance as [re hb s0, s1 | im hb | re ha | im ha][lane]
-    double hb_r[2], hb_i[2], ha_r[2], ha_i[2];
-    auto load_frag = [&](int ci, double* br, double* bi, double* ar, double* ai) {
-        const double* f = dp.p.hfrag + (size_t)ci * 256 + lane;
-#pragma unroll
-        for (int s = 0; s < 2; ++s) {
-            br[s] = __ldg(f + 32 * s);
-            ar[s] = __ldg(f + 32 * (4 + s));
-            if (HK == H_GENERIC) {
-                bi[s] = __ldg(f + 32 * (2 + s));
-                ai[s] = __ldg(f + 32 * (6 + s));
-            } else {
-                bi[s] = ai[s] = 0.0;
-            }
-        }
-    };
-    const double2 g1 = owner ? p.gamma0[e1] : make_double2(0.0, 0.0);
-    const double2 g2 = owner ? p.gamma0[e2] : make_double2(0.0, 0.0);
-    int sli[SLT], slj[SLT], pi[SLT], pj[SLT];
+    // gamma0 of the lane's row elements ([2][32], the same for every warp)
+    if (warp < 2) {
+        const bool in = warp ? ps1 >= 0 : ps0 >= 0;
+        s_g0[threadIdx.x] = in ? p.gamma0[r * N + 2 * t + warp] : make_double2(0.0, 0.0);
+    }
+    int slo[SLT];                                       // record offsets of the slots of state r: their tuple byte
+    int kp[SLT];                                        // table positions of the slots (-1: none)
+    double2 kof[SLT], kgs[SLT], kj[SLT];                // KREG: coefficients of the row elements, of the column elements
 #pragma unroll
     for (int q = 0; q < SLT; ++q) {
-        // diagonal sectors: element 1 = (i1,i1) uses the slots of site i1, element 2 = (i2,i2) those of i2
-        const int a = si, b = diag ? i2 : sj;
-        sli[q] = (owner && q < SL) ? p.slots[a * SL + q] : -1;
-        slj[q] = (owner && q < SL) ? p.slots[b * SL + q] : -1;
-        pi[q] = sli[q] >= 0 ? dp.ct.pos[sli[q]] : 0;
-        pj[q] = slj[q] >= 0 ? dp.ct.pos[slj[q]] : 0;
+        const int sl = (r < N && q < SL) ? p.slots[r * SL + q] : -1;
+        slo[q] = sl >= 0 ? sl : 0;
+        kp[q] = sl >= 0 ? dp.ct.pos[sl] : -1;
+        if (KREG) {
+            const double2* k = dp.ct.khat + kp[q];
+            const double2 z = make_double2(0.0, 0.0);
+            kof[q] = sl >= 0 ? k[dga ? 2 * W : 0] : z;
+            kgs[q] = sl >= 0 ? k[dgb ? 2 * W : 0] : z;
+            kj[q] = sl >= 0 ? k[W] : z;
+            if (ADJ) {
+                kof[q].y = -kof[q].y;
+                kgs[q].y = -kgs[q].y;
+                kj[q].y = -kj[q].y;
+            }
+        }
     }
-    const double2* kap_i1 = s_kh + (diag ? 2 : 0) * W;
-    const double2* kap_j1 = s_kh + 1 * W;
-    const double2* kap_i2 = s_kh + 1 * W;
-    const double2* kap_j2 = s_kh + (diag ? 2 : 0) * W;
+    const double2* kt_of = s_kh + (dga ? 2 : 0) * W;
+    const double2* kt_gs = s_kh + (dgb ? 2 : 0) * W;
+    const double2* kt_j = s_kh + W;
 
     if (lane == 0) {
         mbar_init(&bars[0]);
         mbar_init(&bars[1]);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
+    if (lane < 2) *reinterpret_cast<double2*>(slot + lane * slot_b + zero_off) = make_double2(0.0, 0.0);
     __syncthreads();
 
-    const int64_t nodes = p.nodes;
-    const int64_t stride = (int64_t)gridDim.x * kCtaWarps;
-    int64_t u = (int64_t)blockIdx.x * kCtaWarps + warp;
-    unsigned ph0 = 0u, ph1 = 0u; // mbarrier phase parity of slot 0 / slot 1
+    const unsigned nodes = (unsigned)p.nodes; // at most 2^31 - 1
+    const unsigned stride = gridDim.x * kRowWarps;
+    unsigned u = blockIdx.x * kRowWarps + warp;
     // instance of the current ADO (warp-uniform); its fragments are in hb_* / ha_*
     int ci = (MI && u < nodes) ? __ldg(p.inst + u) : 0;
     // the next ADO's instance, read one iteration ahead of its use so that the
     // instance compare never waits on the load
     int ni_ahead = (MI && u + stride < nodes) ? __ldg(p.inst + u + stride) : ci;
+
+    grid_wait(); // the state and the H tables of a field are written by the kernels before this one
+
+    // operand fragments of H / hbar for k-slice s, k = 2t + s (zero outside the N x N block):
+    //   hb = H(k, r) (B operand of w H), ha = -H(r, k) (A operand of -H w);
+    // packed per instance as [re hb s0, s1 | im hb | re ha | im ha][lane]
+    double hb_r[2], hb_i[2], ha_r[2], ha_i[2];
+    auto load_frag = [&](int c, double* br, double* bi, double* ar, double* ai) {
+        const double* f = dp.p.hfrag + (size_t)c * 256 + lane;
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            br[s] = f[32 * s];
+            if (HK == H_GENERIC) {
+                ar[s] = f[32 * (4 + s)];
+                bi[s] = f[32 * (2 + s)];
+                ai[s] = f[32 * (6 + s)];
+            } else {
+                ar[s] = bi[s] = ai[s] = 0.0;
+            }
+        }
+    };
     load_frag(ci, hb_r, hb_i, ha_r, ha_i);
 
-    auto issue = [&](int64_t v, int sl) {
-        unsigned char* slot = wbase + sl * slot_b;
-        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-        mbar_expect(&bars[sl], tx_bytes);
-        bulk_g2s(slot, p.in + v * (2 * P), tile_b, &bars[sl]);
-        bulk_g2s(slot + nbr_off, p.nbr + v * p.NW, p.NW * 4, &bars[sl]);
-        bulk_g2s(slot + tup_off, p.tup + v * p.TWB, p.TWB, &bars[sl]);
-        bulk_g2s(slot + pss_off, p.pss + v, 16, &bars[sl]);
+    auto issue = [&](unsigned v, unsigned char* dst, uint64_t* bar) {
+        mbar_expect(bar, tile_b + recb);
+        bulk_g2s(dst, p.in + (int64_t)v * (2 * P), tile_b, bar);
+        bulk_g2s(dst + tile_b, p.rec + (int64_t)v * recb, recb, bar);
     };
-    if (u < nodes && lane == 0) issue(u, 0);
-    int cur = 0;
+    // the neighbours of the first slots' batch (QB slots) are read one ADO ahead: vk, vc their indices along K and C,
+    // xo, xg the K neighbours' sectors
+    int vk[QB], vc[QB];
+    double2 xo[QB][2], xg[QB][2];
+    auto load_k = [&](const unsigned char* sl, int q0) {
+        const int2* nb = reinterpret_cast<const int2*>(sl + tile_b);
+#pragma unroll
+        for (int b = 0; b < QB; ++b) {
+            const int2 pm = kp[q0 + b] >= 0 ? nb[slo[q0 + b]] : make_int2(-1, -1);
+            vk[b] = ADJ ? pm.x : pm.y;
+            vc[b] = ADJ ? pm.y : pm.x;
+            const int64_t o = (int64_t)vk[b] * (2 * P);
+            ld256_if(ODD ? vk[b] | no_o : vk[b], in_o + o, xo[b][0], xo[b][1]);
+            ld256_if(ODD ? vk[b] | no_g : vk[b], in_g + o, xg[b][0], xg[b][1]);
+        }
+    };
+    unsigned it = 0; // ADOs done: slot it & 1, mbarrier parity (it >> 1) & 1
     bool failed = false;
-    for (; u < nodes; u += stride) {
-        const int64_t un = u + stride;
-        if (un < nodes && lane == 0) issue(un, cur ^ 1);
+    if (u < nodes) {
+        if (lane == 0) issue(u, slot, bars);
+        if (AHEAD) {
+            if (mbar_wait(bars, 0)) load_k(slot, 0);
+            else failed = true;
+        }
+    }
+    for (; u < nodes && !failed; u += stride, ++it) {
+        const bool more = u + stride < nodes;
+        // (the slot's last readers are behind the __syncwarp of the previous iteration)
+        if (more && lane == 0) issue(u + stride, slot_n, bars + ((it & 1) ^ 1));
         // the next ADO's instance and, when it differs, its fragments (used from the next iteration)
         int ni = ci;
         double nb_r[2], nb_i[2], na_r[2], na_i[2];
-        if (MI && un < nodes) {
+        if (MI && more) {
             ni = ni_ahead;
             if (ni != ci) load_frag(ni, nb_r, nb_i, na_r, na_i);
-            ni_ahead = un + stride < nodes ? __ldg(p.inst + un + stride) : ni;
+            ni_ahead = u + 2 * stride < nodes ? __ldg(p.inst + u + 2 * stride) : ni;
         }
-        if (!mbar_wait(&bars[cur], cur ? ph1 : ph0)) {
-            failed = true;
-            break;
+        if (!AHEAD) {
+            if (!mbar_wait(bars + (it & 1), (it >> 1) & 1)) {
+                failed = true;
+                break;
+            }
+            load_k(slot, 0);
         }
-        if (cur) ph1 ^= 1u; else ph0 ^= 1u;
-        const unsigned char* slot = wbase + cur * slot_b;
-        const double2* tile = reinterpret_cast<const double2*>(slot);
-        const int32_t* nb = reinterpret_cast<const int32_t*>(slot + nbr_off);
         const unsigned char* tu = slot + tup_off;
-        const double2 pss = *reinterpret_cast<const double2*>(slot + pss_off);
 
-        // ---- commutator on the tensor pipe ----
-        double cr0 = 0.0, cr1 = 0.0, ci0 = 0.0, ci1 = 0.0;
-#pragma unroll
-        for (int s = 0; s < 2; ++s) {
-            const int fs = s == 0 ? fs0 : fs1;
-            const int ha = s == 0 ? ha0 : ha1;
-            double2 A = make_double2(0.0, 0.0), B = A;
-            if (fs >= 0) {
-                A = tile[2 * fs + ha];
-                B = (r == 4 * s + t) ? A : tile[2 * fs + (ha ^ 1)];
+        // ---- commutator on the tensor pipe, same term ----
+        double2 of, os, gf, gs; // owned / handed-over sector, first / second half
+        double2 xf, xs;         // the owned sector's own values
+        {
+            const double2 r0 = *reinterpret_cast<const double2*>(slot + ro0);
+            const double2 c0 = *reinterpret_cast<const double2*>(slot + co0);
+            const double2 r1 = *reinterpret_cast<const double2*>(slot + ro1);
+            const double2 c1 = *reinterpret_cast<const double2*>(slot + co1);
+            double2 pss = *reinterpret_cast<const double2*>(slot + pss_off);
+            if (GEN && p.no_same) pss = make_double2(0.0, 0.0);
+            if (ADJ) pss.y = -pss.y;
+            if (!XLATE) {
+                xf = sel2(odd, r1, r0);
+                xs = sel2(odd, c1, c0);
             }
-            dmma(cr0, cr1, A.x, hb_r[s]); // Re(w) Re(H)
-            dmma(ci0, ci1, A.y, hb_r[s]); // Im(w) Re(H)
-            dmma(cr0, cr1, ha_r[s], B.x); // -Re(H) Re(w)
-            dmma(ci0, ci1, ha_r[s], B.y); // -Re(H) Im(w)
-            if (HK == H_GENERIC) {
-                dmma(cr0, cr1, -A.y, hb_i[s]); // -Im(w) Im(H)
-                dmma(ci0, ci1, A.x, hb_i[s]);  //  Re(w) Im(H)
-                dmma(cr0, cr1, -ha_i[s], B.y); // +Im(H) Im(w)
-                dmma(ci0, ci1, ha_i[s], B.x);  // -Im(H) Re(w)
+            double cr0 = 0.0, cr1 = 0.0, ci0 = 0.0, ci1 = 0.0;
+#pragma unroll
+            for (int s = 0; s < 2; ++s) {
+                const double2 A = s ? r1 : r0;
+                const double2 B = s ? c1 : sel2(dga, r0, c0);
+                dmma(cr0, cr1, A.x, hb_r[s]); // Re(w) Re(H)
+                dmma(ci0, ci1, A.y, hb_r[s]); // Im(w) Re(H)
+                if (HK == H_GENERIC) {
+                    dmma(cr0, cr1, ha_r[s], B.x);  // -Re(H) Re(w)
+                    dmma(ci0, ci1, ha_r[s], B.y);  // -Re(H) Im(w)
+                    dmma(cr0, cr1, -A.y, hb_i[s]); // -Im(w) Im(H)
+                    dmma(ci0, ci1, A.x, hb_i[s]);  //  Re(w) Im(H)
+                    dmma(cr0, cr1, -ha_i[s], B.y); // +Im(H) Im(w)
+                    dmma(ci0, ci1, ha_i[s], B.x);  // -Im(H) Re(w)
+                } else { // H(r, k) = H(k, r): the fragment of w H serves both products
+                    dmma(cr0, cr1, hb_r[s], -B.x);
+                    dmma(ci0, ci1, hb_r[s], -B.y);
+                }
+            }
+            // row elements: i * (w H - H w) / hbar and the same term
+            double2 t0 = make_double2(-ci0, cr0), t1 = make_double2(-ci1, cr1);
+            const double2 g0 = s_g0[lane], g1 = s_g0[32 + lane];
+            cmac(t0, make_double2(pss.x + g0.x, pss.y + g0.y), r0);
+            cmac(t1, make_double2(pss.x + g1.x, pss.y + g1.y), r1);
+            of = sel2(odd, t1, t0);
+            gs = sel2(odd, t0, t1);
+            os = gf = make_double2(0.0, 0.0);
+        }
+#pragma unroll
+        for (int q0 = 0; q0 < SLT; q0 += QB) {
+            if (q0 > 0) load_k(slot, q0);
+            // ---- bath terms: K neighbours ----
+#pragma unroll
+            for (int b = 0; b < QB; ++b) {
+                const int q = q0 + b;
+                if (vk[b] >= 0) {
+                    const double2* sq = s_sq + tu[slo[q]];
+                    const double sk = ADJ ? sq->y : sq->x;
+                    auto kap = [&](const double2& reg, const double2* tab) {
+                        const double2 v = KREG ? reg : tab[kp[q]];
+                        return make_double2(v.x * sk, (ADJ && !KREG ? -v.y : v.y) * sk);
+                    };
+                    cmac(of, kap(kof[q], kt_of), xo[b][0]);
+                    cmac(gs, kap(kgs[q], kt_gs), xg[b][1]);
+                    const double2 k = kap(kj[q], kt_j);
+                    if (!dga) cmac(os, k, xo[b][1]);
+                    if (!dgb) cmac(gf, k, xg[b][0]);
+                }
+            }
+            // ---- C neighbours (a diagonal element's terms of its row and column cancel) ----
+#pragma unroll
+            for (int b = 0; b < QB; ++b) {
+                const int64_t o = (int64_t)vc[b] * (2 * P);
+                if (vc[b] >= 0) {
+                    ld256_if(no_co, in_o + o, xo[b][0], xo[b][1]);
+                    ld256_if(no_cg, in_g + o, xg[b][0], xg[b][1]);
+                }
+            }
+#pragma unroll
+            for (int b = 0; b < QB; ++b) {
+                const int q = q0 + b;
+                if (vc[b] >= 0) {
+                    const double2 sq = s_sq[tu[slo[q]]];
+                    const double c = ADJ ? -s_ch[kp[q]] * sq.x : s_ch[kp[q]] * sq.y;
+                    if (!dga) {
+                        of.x = fma(-c, xo[b][0].y, of.x);
+                        of.y = fma(c, xo[b][0].x, of.y);
+                        os.x = fma(c, xo[b][1].y, os.x);
+                        os.y = fma(-c, xo[b][1].x, os.y);
+                    }
+                    if (!dgb) {
+                        gf.x = fma(c, xg[b][0].y, gf.x);
+                        gf.y = fma(-c, xg[b][0].x, gf.y);
+                        gs.x = fma(-c, xg[b][1].y, gs.x);
+                        gs.y = fma(c, xg[b][1].x, gs.y);
+                    }
+                }
             }
         }
-        xch[xw0] = make_double2(cr0, ci0);
-        xch[xw1] = make_double2(cr1, ci1);
-        __syncwarp();
+        // ---- the next ADO's K neighbours: in flight through the exchange, the stores and its commutator ----
+        if (AHEAD && more) {
+            if (mbar_wait(bars + ((it & 1) ^ 1), ((it + 1) >> 1) & 1)) load_k(slot_n, 0);
+            else failed = true;
+        }
+        // ---- the handed-over sector's terms to its owner ----
+        const double2 hf = shfl2(gf, giver), hs = shfl2(gs, giver);
+        const double2 L1 = make_double2(of.x + hf.x, of.y + hf.y);
+        double2 L2 = make_double2(os.x + hs.x, os.y + hs.y);
+        if (ODD && r == N - 1 && dga) L2 = L1; // the padding half mirrors its element
 
         if (owner) {
-            const double2 c1 = xch[xr1], c2 = xch[xr2];
-            // read the halves in a staggered order (conflict-free quarter warps)
-            const int h0 = (lane >> 2) & 1;
-            const double2 sa = tile[2 * lane + h0], sb = tile[2 * lane + (h0 ^ 1)];
-            const double2 s1 = h0 ? sb : sa, s2 = h0 ? sa : sb;
-            double2 L1 = make_double2(-c1.y, c1.x); // i * (w H - H w) / hbar
-            double2 L2 = make_double2(-c2.y, c2.x);
-            cmac(L1, make_double2(pss.x + g1.x, pss.y + g1.y), s1);
-            cmac(L2, make_double2(pss.x + g2.x, pss.y + g2.y), s2);
-
-            // one slot per site: both sides' neighbour rows in one batch (one round trip per ADO)
-            constexpr int SB = SLT == 1 ? 2 : 1;
-#pragma unroll
-            for (int sd0 = 0; sd0 < 2; sd0 += SB) {
-                double2 xp[SB][SLT][2], xm[SB][SLT][2];
-                int nn[SB][SLT];
-#pragma unroll
-                for (int bb = 0; bb < SB; ++bb) {
-                    const int sd = sd0 + bb;
-#pragma unroll
-                    for (int q = 0; q < SLT; ++q) {
-                        const int sl = sd == 0 ? sli[q] : slj[q];
-                        // diagonal elements: the plus terms of L cancel (the minus terms of L^H)
-                        const int2 pm = sl >= 0 ? reinterpret_cast<const int2*>(nb)[sl] : make_int2(-1, -1);
-                        const int32_t vp = (ADJ || !diag) ? pm.x : -1;
-                        const int32_t vm = (!ADJ || !diag) ? pm.y : -1;
-                        nn[bb][q] = sl >= 0 ? tu[sl] : 0;
-                        xp[bb][q][0] = xp[bb][q][1] = xm[bb][q][0] = xm[bb][q][1] = make_double2(0.0, 0.0);
-                        if (vp >= 0) ld256(p.in + (int64_t)vp * (2 * P) + 2 * lane, xp[bb][q][0], xp[bb][q][1]);
-                        if (vm >= 0) ld256(p.in + (int64_t)vm * (2 * P) + 2 * lane, xm[bb][q][0], xm[bb][q][1]);
-                    }
-                }
-#pragma unroll
-                for (int bb = 0; bb < SB; ++bb) {
-                    const int sd = sd0 + bb;
-#pragma unroll
-                    for (int q = 0; q < SLT; ++q) {
-                        const int sl = sd == 0 ? sli[q] : slj[q];
-                        if (sl < 0) continue;
-                        const int ps = sd == 0 ? pi[q] : pj[q];
-                        const double2 sqp = s_sq[nn[bb][q]];
-                        const double sq_lo = sqp.x, sq_hi = sqp.y;
-                        // L:   i-coefficient term on the plus neighbour (chat sqrt(n+1)),
-                        //      complex term on the minus neighbour (khat sqrt(n))
-                        // L^H: i-coefficient term on the minus neighbour (-chat sqrt(n)),
-                        //      complex term on the plus neighbour (conj(khat) sqrt(n+1))
-                        const double c = diag ? 0.0 : (ADJ ? -s_ch[ps] * sq_lo : s_ch[ps] * sq_hi);
-                        const double sk = ADJ ? sq_hi : sq_lo;
-                        const double2 t1 = ADJ ? xm[bb][q][0] : xp[bb][q][0], t2 = ADJ ? xm[bb][q][1] : xp[bb][q][1];
-                        const double2 k1 = ADJ ? xp[bb][q][0] : xm[bb][q][0], k2 = ADJ ? xp[bb][q][1] : xm[bb][q][1];
-                        // the complex-coefficient neighbour scales as sqrt(n) (sqrt(n+1) for L^H); fold it in
-                        const double2 m1 = make_double2(k1.x * sk, k1.y * sk);
-                        const double2 m2 = make_double2(k2.x * sk, k2.y * sk);
-                        auto kap = [&](const double2* tab) {
-                            const double2 v = tab[ps];
-                            return ADJ ? make_double2(v.x, -v.y) : v;
-                        };
-                        if (sd == 0) {
-                            L1.x = fma(-c, t1.y, L1.x);
-                            L1.y = fma(c, t1.x, L1.y);
-                            L2.x = fma(c, t2.y, L2.x);
-                            L2.y = fma(-c, t2.x, L2.y);
-                            cmac(L1, kap(kap_i1), m1);
-                            if (!diag) cmac(L2, kap(kap_i2), m2);
-                        } else {
-                            L1.x = fma(c, t1.y, L1.x);
-                            L1.y = fma(-c, t1.x, L1.y);
-                            L2.x = fma(-c, t2.y, L2.x);
-                            L2.y = fma(c, t2.x, L2.y);
-                            if (!diag) cmac(L1, kap(kap_j1), m1);
-                            cmac(L2, kap(kap_j2), m2);
-                        }
-                    }
-                }
+            const int64_t off = (int64_t)u * (2 * P) + 2 * pso;
+            if (XLATE) {
+                xf = *reinterpret_cast<const double2*>(slot + (odd ? ro1 : ro0));
+                xs = *reinterpret_cast<const double2*>(slot + (odd ? co1 : co0));
             }
-
-            const int64_t off = u * (2 * P) + 2 * lane;
-            double2 x1 = s1, x2 = s2;
-            if (p.y) ld256_cg(p.y + off, x1, x2);
-            double2 o1 = make_double2(p.alpha.x * x1.x - p.alpha.y * x1.y, p.alpha.x * x1.y + p.alpha.y * x1.x);
-            double2 o2 = make_double2(p.alpha.x * x2.x - p.alpha.y * x2.y, p.alpha.x * x2.y + p.alpha.y * x2.x);
+            double2 o1 = xf, o2 = xs;
+            if (GEN) {
+                if (p.y) ld256_cg(p.y + off, o1, o2);
+                if (!p.use_x) o1 = o2 = make_double2(0.0, 0.0);
+            }
             cmac(o1, p.beta, L1);
             cmac(o2, p.beta, L2);
             st256_cs(p.out + off, o1, o2);
-            if (p.use_acc) {
-                double2 a1 = s1, a2 = s2;
+            if (GEN && p.use_acc) {
+                double2 a1 = xf, a2 = xs;
                 if (!p.acc_init) ld256_cg(p.acc + off, a1, a2);
                 cmac(a1, p.acc_beta, L1);
                 cmac(a2, p.acc_beta, L2);
@@ -589,7 +729,9 @@ __global__ void __launch_bounds__(kCtaWarps * 32, 2) heom_dmma_stage(const DmmaP
             }
         }
         __syncwarp();
-        cur ^= 1;
+        unsigned char* const sw = slot;
+        slot = slot_n;
+        slot_n = sw;
         if (MI && ni != ci) {
 #pragma unroll
             for (int s = 0; s < 2; ++s) {
@@ -601,11 +743,9 @@ __global__ void __launch_bounds__(kCtaWarps * 32, 2) heom_dmma_stage(const DmmaP
             ci = ni;
         }
     }
-    if (failed) {
-        if (lane == 0) atomicExch(dp.err, 1);
-        // let copies still in flight land before the warp leaves (bounded)
-        mbar_wait(&bars[cur ^ 1], cur ? ph0 : ph1);
-    }
+    // a warp whose wait expired flags the launch as failed and leaves; every copy it issued was either waited
+    // for or is the one whose wait has just run to its limit
+    if (failed && lane == 0) atomicExch(dp.err, 1);
 }
 
 // ---------------------------------------------------------------------------
@@ -663,11 +803,9 @@ __device__ __forceinline__ void prefetch_ado(unsigned char* slot, const PairPara
         cp_async16(tile + tile_pos(N, i1, j1), src + 2 * lt);
         cp_async16(tile + tile_pos(N, i2, j2), src + 2 * lt + 1);
     }
-    int32_t* nb = reinterpret_cast<int32_t*>(slot + L.nbr_off);
-    for (int q = lt * 4; q < p.NW; q += tt * 4) cp_async16(nb + q, p.nbr + u * p.NW + q);
-    unsigned char* tu = slot + L.tup_off;
-    for (int q = lt * 16; q < p.TWB; q += tt * 16) cp_async16(tu + q, p.tup + u * p.TWB + q);
-    if (lt == 0) cp_async16(slot + L.pss_off, p.pss + u);
+    // the record's parts lie back to back in the slot
+    const int recb = rec_bytes(p.NW, p.TWB);
+    for (int q = lt * 16; q < recb; q += tt * 16) cp_async16(slot + L.nbr_off + q, p.rec + u * recb + q);
 }
 
 // ADJ: the adjoint operator L^H (see heom_dmma_stage).  The bath
@@ -675,7 +813,7 @@ __device__ __forceinline__ void prefetch_ado(unsigned char* slot, const PairPara
 // (three CTAs per SM where at most two slots per state keep the register
 // demand low enough; two otherwise)
 template <int N, int HK, int SLT, bool ADJ>
-__global__ void __launch_bounds__(kCtaWarps * 32, SLT <= 2 ? 3 : 2) heom_pair_stage(const DmmaParams dp)
+__global__ void __launch_bounds__(kCtaWarps * 32, SLT <= 2 ? 3 : 2) heom_pair_stage(const __grid_constant__ DmmaParams dp)
 {
     static_assert(N > 8 && N <= 16, "team kernel handles N = 9..16");
     constexpr int P = pairs_of(N);
@@ -688,6 +826,7 @@ __global__ void __launch_bounds__(kCtaWarps * 32, SLT <= 2 ? 3 : 2) heom_pair_st
     const PairParams& p = dp.p;
     const PairSmem L = pair_smem_layout(N, p.W, p.NW, p.TWB, p.LS);
     const int W = p.W, LS = p.LS, SL = p.SL;
+    grid_launch_dependents();
 
     double2* s_kh = reinterpret_cast<double2*>(smem);      // 3 * W
     double2* s_sq = s_kh + 3 * W;                           // LS + 1: (sqrt(n), sqrt(n+1))
@@ -726,6 +865,7 @@ __global__ void __launch_bounds__(kCtaWarps * 32, SLT <= 2 ? 3 : 2) heom_pair_st
 
     __syncthreads();
     if (team >= TEAMS) return;
+    grid_wait(); // the state and the H tables of a field are written by the kernels before this one
 
     const int64_t nodes = p.nodes;
     const int64_t stride = (int64_t)gridDim.x * TEAMS;
@@ -760,15 +900,15 @@ __global__ void __launch_bounds__(kCtaWarps * 32, SLT <= 2 ? 3 : 2) heom_pair_st
                 const double2 z = make_double2(0.0, 0.0);
                 const double2 A = (ra < N && ka < N) ? t[tile_pos(N, ra, ka)] : z;
                 const double2 B = (ka < N && cb < N) ? t[tile_pos(N, ka, cb)] : z;
-                const double hbr = __ldg(fr + frag_index(N, 0, J, s, lane));
-                const double har = __ldg(fr + frag_index(N, 2, I, s, lane));
+                const double hbr = fr[frag_index(N, 0, J, s, lane)];
+                const double har = fr[frag_index(N, 2, I, s, lane)];
                 dmma(cr0, cr1, A.x, hbr); // Re(w) Re(H)
                 dmma(ci0, ci1, A.y, hbr); // Im(w) Re(H)
                 dmma(cr0, cr1, har, B.x); // -Re(H) Re(w)
                 dmma(ci0, ci1, har, B.y); // -Re(H) Im(w)
                 if (HK == H_GENERIC) {
-                    const double hbi = __ldg(fr + frag_index(N, 1, J, s, lane));
-                    const double hai = __ldg(fr + frag_index(N, 3, I, s, lane));
+                    const double hbi = fr[frag_index(N, 1, J, s, lane)];
+                    const double hai = fr[frag_index(N, 3, I, s, lane)];
                     dmma(cr0, cr1, -A.y, hbi); // -Im(w) Im(H)
                     dmma(ci0, ci1, A.x, hbi);  //  Re(w) Im(H)
                     dmma(cr0, cr1, -hai, B.y); // +Im(H) Im(w)
@@ -789,7 +929,9 @@ __global__ void __launch_bounds__(kCtaWarps * 32, SLT <= 2 ? 3 : 2) heom_pair_st
         if (active) {
             const int32_t* nb = reinterpret_cast<const int32_t*>(slot + L.nbr_off);
             const unsigned char* tu = slot + L.tup_off;
-            const double2 pss = *reinterpret_cast<const double2*>(slot + L.pss_off);
+            double2 pss = *reinterpret_cast<const double2*>(slot + L.pss_off);
+            if (p.no_same) pss = make_double2(0.0, 0.0);
+            if (ADJ) pss.y = -pss.y;
             s1 = t[tile_pos(N, i1, j1)];
             s2 = t[tile_pos(N, i2, j2)];
 
@@ -878,8 +1020,7 @@ __global__ void __launch_bounds__(kCtaWarps * 32, SLT <= 2 ? 3 : 2) heom_pair_st
             const int64_t off = u * (2 * P) + 2 * lt;
             double2 x1 = s1, x2 = s2;
             if (p.y) ld256_cg(p.y + off, x1, x2);
-            double2 r1 = make_double2(p.alpha.x * x1.x - p.alpha.y * x1.y, p.alpha.x * x1.y + p.alpha.y * x1.x);
-            double2 r2 = make_double2(p.alpha.x * x2.x - p.alpha.y * x2.y, p.alpha.x * x2.y + p.alpha.y * x2.x);
+            double2 r1 = p.use_x ? x1 : make_double2(0.0, 0.0), r2 = p.use_x ? x2 : make_double2(0.0, 0.0);
             cmac(r1, p.beta, L1);
             cmac(r2, p.beta, L2);
             st256_cs(p.out + off, r1, r2);
@@ -1034,8 +1175,7 @@ __global__ void heom_write_top(double2* __restrict__ y, const double2* __restric
 struct GradParams {
     const double2* __restrict__ a;     // adjoint (pair layout, internal order)
     const double2* __restrict__ w;     // forward stage input
-    const int32_t* __restrict__ nbr;   // [nodes][NW] (plus, minus) of every slot
-    const uint8_t* __restrict__ tup;   // [nodes][TWB]
+    const unsigned char* __restrict__ rec; // [nodes] records: (plus, minus) of every slot, tuple bytes
     const int16_t* __restrict__ pe;    // [2P] element indices of the sector halves
     const int16_t* __restrict__ slots; // [N][SL] slot ids of each state, -1 padded
     const double* __restrict__ dpss;   // [nodes] d pf_same_sum / d gamma (real)
@@ -1082,8 +1222,8 @@ __global__ void __launch_bounds__(kCtaWarps * 32) heom_adjoint_grad(const GradPa
     const int inst = blockIdx.x / g.blocks_per_inst, jb = blockIdx.x - inst * g.blocks_per_inst;
     const int64_t stride = (int64_t)g.blocks_per_inst * kCtaWarps, end = g.inst_base[inst + 1];
     for (int64_t u = g.inst_base[inst] + (int64_t)jb * kCtaWarps + warp; u < end; u += stride) {
-        const int32_t* nb = g.nbr + u * g.NW;
-        const uint8_t* tu = g.tup + u * g.TWB;
+        const unsigned char* nb = g.rec + u * rec_bytes(g.NW, g.TWB);
+        const unsigned char* tu = nb + g.NW * 4;
         const double dps = g.dpss[u];
         for (int p = lane; p < P; p += 32) {
             const int e1 = g.pe[2 * p], e2 = g.pe[2 * p + 1];
@@ -1308,7 +1448,7 @@ __global__ void heom_field_tables(const FieldParams f)
                 for (int q = threadIdx.x; q < fd; q += blockDim.x) {
                     // operand fragments as in the host tables ([kind][block][k-slice][lane], frag_index)
                     const int l = q & 31, part = q >> 5, sl = part % ns, b = (part / ns) % nb, kind = part / (ns * nb);
-                    const int r = 8 * b + (l >> 2), c = 4 * sl + (l & 3);
+                    const int r = 8 * b + (l >> 2), c = frag_col(N, sl, l & 3);
                     double v = 0.0;
                     if (r < N && c < N) {
                         const double2 hcr = hs[c * N + r], hrc = hs[r * N + c];

@@ -18,7 +18,7 @@
 namespace heomk {
 
 struct LockParams {
-    PairParams p;     // in/out/y/acc in the lockstep layout; nbr/tup/pss rows of one instance; hfrag [K][256]
+    PairParams p;     // in/out/y/acc in the lockstep layout; records of one instance; hfrag [K][256]
     LaneTab lt;
     CoefTabs ct;
     int K;            // instances
@@ -30,16 +30,16 @@ constexpr int kLockWarps = 8;
 // one slot of one site at the current ADO: its neighbour rows and coefficients
 struct __align__(16) LockSlot {
     int64_t op, om;   // byte offsets of the rows of ADO n + e (plus) and n - e (minus); -1: absent
-    double c, sm;     // plus-side coefficient chat * sqrt(n + 1), minus-side scale sqrt(n)
-    double2 kap[3];   // the three kappa-hat values of the slot's mode
-    int present, pad[3];
+    double2 kap[3];   // minus-side coefficients: the three kappa-hat values of the slot times sqrt(n)
+    double c;         // plus-side coefficient chat * sqrt(n + 1)
+    double pad;
 };
-// one pair sector: its sites and same-term values
+// one pair sector, in the order in which the warps take them: its sites and same-term values
 struct __align__(16) LockSector {
-    int sa, sb, diag, pad; // sites of side 0 and side 1 (element i1, then j1 or, diagonal, i2)
+    int sa, sb, diag, ps;  // sites of side 0 and side 1 (element i1, then j1 or, diagonal, i2); the sector
     double2 g1, g2;        // gamma0 of its two elements
 };
-__host__ __device__ inline int lock_row_bytes(int NW, int TWB) { return ((NW * 4 + 15) & ~15) + ((TWB + 15) & ~15) + 16; }
+__host__ __device__ inline int lock_row_bytes(int NW, int TWB) { return rec_bytes(NW, TWB); }
 __host__ inline size_t lockstep_smem_bytes(int P, int W, int NW, int TWB, int LS)
 {
     return (size_t)dmma_lut_bytes(W, LS) + 2 * (size_t)P * 32 * 32 /* two tiles */ + 32 * 32 * 32 /* commutators */ +
@@ -47,27 +47,14 @@ __host__ inline size_t lockstep_smem_bytes(int P, int W, int NW, int TWB, int LS
            2 * (size_t)lock_row_bytes(NW, TWB);
 }
 
-// 32 bytes at base + off (bytes) when off >= 0, zeros otherwise: the test, the address and the
-// load in one asm block
+// 32 bytes at base + off (bytes) when off >= 0; otherwise a and b keep what they hold: the test, the
+// address and the load in one asm block
 __device__ __forceinline__ void ld256_at(const double2* base, int64_t off, double2& a, double2& b)
 {
     asm("{\n .reg .pred q;\n .reg .b64 ad;\n setp.ge.s64 q, %5, 0;\n add.s64 ad, %4, %5;\n"
-        " mov.f64 %0, 0d0000000000000000;\n mov.f64 %1, 0d0000000000000000;\n"
-        " mov.f64 %2, 0d0000000000000000;\n mov.f64 %3, 0d0000000000000000;\n"
-        " @q ld.global.nc.v4.f64 {%0,%1,%2,%3}, [ad];\n}\n"
-        : "=d"(a.x), "=d"(a.y), "=d"(b.x), "=d"(b.y)
+        " @q ld.global.v4.f64 {%0,%1,%2,%3}, [ad];\n}\n"
+        : "+d"(a.x), "+d"(a.y), "+d"(b.x), "+d"(b.y)
         : "l"(base), "l"(off));
-}
-// as ld256_at, and only when skip == 0
-__device__ __forceinline__ void ld256_at_unless(const double2* base, int64_t off, unsigned skip, double2& a, double2& b)
-{
-    asm("{\n .reg .pred q;\n .reg .b64 ad;\n setp.ge.s64 q, %5, 0;\n setp.eq.and.u32 q, %6, 0, q;\n"
-        " add.s64 ad, %4, %5;\n"
-        " mov.f64 %0, 0d0000000000000000;\n mov.f64 %1, 0d0000000000000000;\n"
-        " mov.f64 %2, 0d0000000000000000;\n mov.f64 %3, 0d0000000000000000;\n"
-        " @q ld.global.nc.v4.f64 {%0,%1,%2,%3}, [ad];\n}\n"
-        : "=d"(a.x), "=d"(a.y), "=d"(b.x), "=d"(b.y)
-        : "l"(base), "l"(off), "r"(skip));
 }
 // 32 bytes through the coherent path, schedulable: the stage kernel stores to the same address only
 // values computed from the loaded ones, which orders the load first
@@ -87,16 +74,18 @@ __device__ __forceinline__ void ld256_co(const double2* src, double2& a, double2
 // instance; every global read of a sector (the neighbour rows of both sides,
 // y and acc) is issued, predicated, before its arithmetic.
 template <int N, int HK, int SLT>
-__global__ void __launch_bounds__(kLockWarps * 32, 2) heom_lockstep_stage(const LockParams lp)
+__global__ void __launch_bounds__(kLockWarps * 32, 2) heom_lockstep_stage(const __grid_constant__ LockParams lp)
 {
     static_assert(N <= 8 && N * SLT <= 32, "lockstep stage handles N <= 8");
     constexpr int P = pairs_of(N);
     constexpr int IPW = 32 / kLockWarps;  // instances per warp in phase A
     constexpr int SB = SLT <= 1 ? 2 : 1; // sides whose neighbour rows are read in one batch
+    constexpr int QB = SLT < 2 ? SLT : 2; // slots read in one batch
     constexpr int TW = kLockWarps - 1;   // the warp that builds the site table
     const PairParams& p = lp.p;
     extern __shared__ __align__(128) unsigned char smem[];
     const int W = p.W, LS = p.LS, SL = p.SL;
+    grid_launch_dependents();
     double2* s_kh = reinterpret_cast<double2*>(smem);
     double2* s_sq = s_kh + 3 * W;
     double* s_ch = reinterpret_cast<double*>(s_sq + LS + 1);
@@ -121,13 +110,13 @@ __global__ void __launch_bounds__(kLockWarps * 32, 2) heom_lockstep_stage(const 
     const int64_t PK2 = (int64_t)P * Kp * 2; // double2 elements of one ADO (all instances)
 
     if (threadIdx.x < P) {
-        const int e1 = lp.lt.e1[threadIdx.x], e2 = lp.lt.e2[threadIdx.x];
+        const int ps = lp.lt.ord[threadIdx.x], e1 = lp.lt.e1[ps], e2 = lp.lt.e2[ps];
         const int i1 = e1 / N, j1 = e1 - i1 * N, i2 = e2 / N;
         LockSector sc;
         sc.sa = i1;
         sc.diag = i1 == j1;
         sc.sb = sc.diag ? i2 : j1;
-        sc.pad = 0;
+        sc.ps = ps;
         sc.g1 = p.gamma0[e1];
         sc.g2 = p.gamma0[e2];
         sectors[threadIdx.x] = sc;
@@ -144,10 +133,10 @@ __global__ void __launch_bounds__(kLockWarps * 32, 2) heom_lockstep_stage(const 
     }
 
     const bool owner = lane < P;
-    const int ae1 = owner ? lp.lt.e1[lane] : 0, ae2 = owner ? lp.lt.e2[lane] : 0;
+    const int ae1 = opaque(owner ? lp.lt.e1[lane] : 0), ae2 = opaque(owner ? lp.lt.e2[lane] : 0);
     const int ai1 = ae1 / N, aj1 = ae1 - ai1 * N, ai2 = ae2 / N, aj2 = ae2 - ai2 * N;
-    const int fs0 = lp.lt.fs[lane][0], fs1 = lp.lt.fs[lane][1];
-    const int ha0 = lp.lt.ha[lane][0], ha1 = lp.lt.ha[lane][1];
+    const int fs0 = opaque(lp.lt.fs[lane][0]), fs1 = opaque(lp.lt.fs[lane][1]);
+    const int ha0 = opaque(lp.lt.ha[lane][0]), ha1 = opaque(lp.lt.ha[lane][1]);
     const int r = lane >> 2, t = lane & 3;
     const int xr1 = 8 * ai1 + (aj1 ^ swz(ai1)), xr2 = 8 * ai2 + (aj2 ^ swz(ai2));
     const int xw0 = 8 * r + ((2 * t) ^ swz(r)), xw1 = 8 * r + ((2 * t + 1) ^ swz(r));
@@ -165,7 +154,7 @@ __global__ void __launch_bounds__(kLockWarps * 32, 2) heom_lockstep_stage(const 
         const int fs = s == 0 ? fs0 : fs1, ha = s == 0 ? ha0 : ha1;
         const int row = fs >= 0 ? (fs * 32 + (warp ^ (fs & 3))) * 2 : 0;
         oa[s] = fs >= 0 ? row + (ha ^ hw) : 0;
-        ob[s] = fs >= 0 ? (r == 4 * s + t ? row + (ha ^ hw) : row + (ha ^ 1 ^ hw)) : 0; // diagonal: its own transpose
+        ob[s] = fs >= 0 ? (r == 2 * t + s ? row + (ha ^ hw) : row + (ha ^ 1 ^ hw)) : 0; // diagonal: its own transpose
     }
     const int oc = (lane * 32 + (warp ^ (lane & 3))) * 2; // this lane's commutator row (lanes >= P: unused rows)
     // its two commutator stores: first position (lane >> 2) & 1, whichever half lives there
@@ -187,16 +176,14 @@ __global__ void __launch_bounds__(kLockWarps * 32, 2) heom_lockstep_stage(const 
         const double2* src = p.in + u * PK2 + src0;
         for (int pp = pp0; pp < P; pp += 4, dst += 4 * 64, src += 8 * Kp) cp_async16(dst, src);
         unsigned char* rows = rows0 + b * rowb;
-        for (int q = threadIdx.x * 4; q < p.NW; q += blockDim.x * 4)
-            cp_async16(reinterpret_cast<int32_t*>(rows) + q, p.nbr + u * p.NW + q);
-        unsigned char* tu = rows + ((p.NW * 4 + 15) & ~15);
-        for (int q = threadIdx.x * 16; q < p.TWB; q += blockDim.x * 16) cp_async16(tu + q, p.tup + u * p.TWB + q);
-        if (threadIdx.x == 0) cp_async16(tu + ((p.TWB + 15) & ~15), p.pss + u);
+        const int recb = rec_bytes(p.NW, p.TWB);
+        for (int q = threadIdx.x * 16; q < recb; q += blockDim.x * 16) cp_async16(rows + q, p.rec + u * recb + q);
     };
 
-    const int k = kb * 32 + lane;
-    const bool live = k < lp.K;
+    const int kl = kb * 32 + lane;
+    const bool live = kl < lp.K;
     const bool read_acc = p.use_acc && !p.acc_init;
+    grid_wait(); // the state is written by the kernels before this one
     int64_t u = blockIdx.x / kblocks;
     int cur = 0;
     if (u < lp.nodes) prefetch(u, 0);
@@ -213,22 +200,21 @@ __global__ void __launch_bounds__(kLockWarps * 32, 2) heom_lockstep_stage(const 
         // ---- the site table of this ADO ----
         if (warp == TW && lane < N * SLT) {
             LockSlot e;
-            e.pad[0] = e.pad[1] = e.pad[2] = 0;
+            e.pad = 0.0;
             if (tsl >= 0) {
                 const int2 pm = reinterpret_cast<const int2*>(rows)[tsl];
                 const double2 sqp = s_sq[tu[tsl]];
                 e.op = pm.x >= 0 ? pm.x * PK2 * 16 : -1;
                 e.om = pm.y >= 0 ? pm.y * PK2 * 16 : -1;
-                e.present = 1;
                 e.c = s_ch[tpos] * sqp.y;
-                e.sm = sqp.x;
-                e.kap[0] = s_kh[tpos];
-                e.kap[1] = s_kh[W + tpos];
-                e.kap[2] = s_kh[2 * W + tpos];
+#pragma unroll
+                for (int q = 0; q < 3; ++q) {
+                    const double2 v = s_kh[q * W + tpos];
+                    e.kap[q] = make_double2(v.x * sqp.x, v.y * sqp.x);
+                }
             } else {
                 e.op = e.om = -1;
-                e.present = 0;
-                e.c = e.sm = 0.0;
+                e.c = 0.0;
                 e.kap[0] = e.kap[1] = e.kap[2] = make_double2(0.0, 0.0);
             }
             slots[lane] = e;
@@ -299,78 +285,84 @@ __global__ void __launch_bounds__(kLockWarps * 32, 2) heom_lockstep_stage(const 
         __syncthreads();
 
         // ---- B: per sector, lane = instance ----
-        for (int ps = warp; ps < P; ps += kLockWarps) {
-            const LockSector sc = sectors[ps];
+        for (int k = warp; k < P; k += kLockWarps) {
+            const LockSector sc = sectors[k];
+            const int ps = sc.ps;
             const bool diag = sc.diag != 0;
-            const int64_t lofs = ((int64_t)ps * Kp + k) * 2; // this lane's sector within an ADO
+            const int64_t lofs = ((int64_t)ps * Kp + kl) * 2; // this lane's sector within an ADO
             const double2* in_l = p.in + lofs;
             const int64_t off = u * PK2 + lofs;
-            double2 x1, x2, a1, a2;
-            double2 L1, L2, s1, s2;
+            double2 x1, x2, a1, a2, s1, s2;
+            // terms of side 0 (the first half's row) and of side 1, for both halves of the sector; either half's
+            // own row starts with its commutator and same term
+            double2 A[2][2];
+            A[0][1] = A[1][0] = make_double2(0.0, 0.0);
 #pragma unroll
             for (int sd0 = 0; sd0 < 2; sd0 += SB) {
-                // neighbour rows of SB sides (absent rows: no load, zeros)
-                double2 xp[SB][SLT][2], xm[SB][SLT][2];
 #pragma unroll
-                for (int b = 0; b < SB; ++b) {
-                    const LockSlot* es = slots + ((sd0 + b) == 0 ? sc.sa : sc.sb) * SLT;
+                for (int q0 = 0; q0 < SLT; q0 += QB) {
+                    // neighbour rows of SB sides and QB slots (absent rows: no load, zeros)
+                    double2 xp[SB][QB][2], xm[SB][QB][2];
 #pragma unroll
-                    for (int q = 0; q < SLT; ++q) {
-                        const longlong2 o = *reinterpret_cast<const longlong2*>(&es[q].op);
-                        ld256_at_unless(in_l, o.x, sc.diag, xp[b][q][0], xp[b][q][1]);
-                        ld256_at(in_l, o.y, xm[b][q][0], xm[b][q][1]);
+                    for (int b = 0; b < SB; ++b) {
+                        const LockSlot* es = slots + ((sd0 + b) == 0 ? sc.sa : sc.sb) * SLT + q0;
+#pragma unroll
+                        for (int q = 0; q < QB; ++q) {
+                            const longlong2 o = *reinterpret_cast<const longlong2*>(&es[q].op);
+                            ld256_at(in_l, o.y, xm[b][q][0], xm[b][q][1]);
+                            ld256_at(in_l, diag ? -1 : o.x, xp[b][q][0], xp[b][q][1]);
+                        }
                     }
-                }
-                if (sd0 == 0) {
-                    if (p.y) ld256_co(p.y + off, x1, x2); // kernel parameters: uniform branches
-                    if (read_acc) ld256_co(p.acc + off, a1, a2);
-                    const int col = (ps * 32 + (lane ^ (ps & 3))) * 2;
-                    s1 = tile[col + hk];
-                    s2 = tile[col + (hk ^ 1)];
-                    const double2 c1 = ctile[col + hk], c2 = ctile[col + (hk ^ 1)];
-                    L1 = make_double2(-c1.y, c1.x); // i * (w H - H w) / hbar
-                    L2 = make_double2(-c2.y, c2.x);
-                    cmac(L1, make_double2(pss.x + sc.g1.x, pss.y + sc.g1.y), s1);
-                    cmac(L2, make_double2(pss.x + sc.g2.x, pss.y + sc.g2.y), s2);
-                }
+                    if (sd0 == 0 && q0 == 0) {
+                        if (p.y) ld256_co(p.y + off, x1, x2); // kernel parameters: uniform branches
+                        if (read_acc) ld256_co(p.acc + off, a1, a2);
+                        const int col = (ps * 32 + (lane ^ (ps & 3))) * 2;
+                        s1 = tile[col + hk];
+                        s2 = tile[col + (hk ^ 1)];
+                        const double2 c1 = ctile[col + hk], c2 = ctile[col + (hk ^ 1)];
+                        A[0][0] = make_double2(-c1.y, c1.x); // i * (w H - H w) / hbar
+                        A[1][1] = make_double2(-c2.y, c2.x);
+                        cmac(A[0][0], make_double2(pss.x + sc.g1.x, pss.y + sc.g1.y), s1);
+                        cmac(A[1][1], make_double2(pss.x + sc.g2.x, pss.y + sc.g2.y), s2);
+                    }
 #pragma unroll
-                for (int b = 0; b < SB; ++b) {
-                    const int sd = sd0 + b;
-                    const LockSlot* es = slots + (sd == 0 ? sc.sa : sc.sb) * SLT;
+                    for (int b = 0; b < SB; ++b) {
+                        const int sd = sd0 + b;
+                        const LockSlot* es = slots + (sd == 0 ? sc.sa : sc.sb) * SLT + q0;
+                        // minus neighbours of the batch, then its plus neighbours (heom_dmma_stage's order)
 #pragma unroll
-                    for (int q = 0; q < SLT; ++q) {
-                        if (!es[q].present) continue; // warp-uniform
-                        const double2 cs = *reinterpret_cast<const double2*>(&es[q].c);
-                        const double c = diag ? 0.0 : cs.x;
-                        const double sm = cs.y;
-                        const double2 m1 = make_double2(xm[b][q][0].x * sm, xm[b][q][0].y * sm);
-                        const double2 m2 = make_double2(xm[b][q][1].x * sm, xm[b][q][1].y * sm);
-                        const double2 t1 = xp[b][q][0], t2 = xp[b][q][1];
-                        const double2 kd = es[q].kap[diag ? 2 : 0], k1 = es[q].kap[1];
-                        if (sd == 0) {
-                            L1.x = fma(-c, t1.y, L1.x);
-                            L1.y = fma(c, t1.x, L1.y);
-                            L2.x = fma(c, t2.y, L2.x);
-                            L2.y = fma(-c, t2.x, L2.y);
-                            cmac(L1, kd, m1);
-                            if (!diag) cmac(L2, k1, m2);
-                        } else {
-                            L1.x = fma(c, t1.y, L1.x);
-                            L1.y = fma(-c, t1.x, L1.y);
-                            L2.x = fma(-c, t2.y, L2.x);
-                            L2.y = fma(c, t2.x, L2.y);
-                            if (!diag) cmac(L1, k1, m1);
-                            cmac(L2, kd, m2);
+                        for (int q = 0; q < QB; ++q) {
+                            if (es[q].om < 0) continue; // warp-uniform
+                            const double2 kd = es[q].kap[diag ? 2 : 0], kj = es[q].kap[1];
+                            if (sd == 0) {
+                                cmac(A[0][0], kd, xm[b][q][0]);
+                                if (!diag) cmac(A[0][1], kj, xm[b][q][1]);
+                            } else {
+                                if (!diag) cmac(A[1][0], kj, xm[b][q][0]);
+                                cmac(A[1][1], kd, xm[b][q][1]);
+                            }
+                        }
+                        if (diag) continue; // the plus terms of a diagonal element's row and column cancel
+#pragma unroll
+                        for (int q = 0; q < QB; ++q) {
+                            if (es[q].op < 0) continue;
+                            const double c = sd == 0 ? es[q].c : -es[q].c;
+                            const double2 t1 = xp[b][q][0], t2 = xp[b][q][1];
+                            A[sd][0].x = fma(-c, t1.y, A[sd][0].x);
+                            A[sd][0].y = fma(c, t1.x, A[sd][0].y);
+                            A[sd][1].x = fma(c, t2.y, A[sd][1].x);
+                            A[sd][1].y = fma(-c, t2.x, A[sd][1].y);
                         }
                     }
                 }
             }
+            const double2 L1 = make_double2(A[0][0].x + A[1][0].x, A[0][0].y + A[1][0].y);
+            const double2 L2 = make_double2(A[0][1].x + A[1][1].x, A[0][1].y + A[1][1].y);
             if (!p.y) {
                 x1 = s1;
                 x2 = s2;
             }
-            double2 o1 = make_double2(p.alpha.x * x1.x - p.alpha.y * x1.y, p.alpha.x * x1.y + p.alpha.y * x1.x);
-            double2 o2 = make_double2(p.alpha.x * x2.x - p.alpha.y * x2.y, p.alpha.x * x2.y + p.alpha.y * x2.x);
+            double2 o1 = p.use_x ? x1 : make_double2(0.0, 0.0), o2 = p.use_x ? x2 : make_double2(0.0, 0.0);
             cmac(o1, p.beta, L1);
             cmac(o2, p.beta, L2);
             st256_cs_if(live, p.out + off, o1, o2);

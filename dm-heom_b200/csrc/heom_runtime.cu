@@ -24,6 +24,7 @@
 
 namespace {
 #include "pair_tables.inc"
+#include "row_tables.inc"
 }
 
 using heomk::PairParams;
@@ -129,38 +130,41 @@ stage_fn_t pick_stage(int n, int hk, int slt, bool adj)
     }
 }
 
-template <int N, int HK, bool MI, bool ADJ>
+// gen: every write mode, or the product form's out = in + beta L only
+template <int N, int HK, bool MI, bool ADJ, bool GEN>
 dmma_fn_t pick_dslt(int slt)
 {
     switch (slt) {
-    case 1: return heomk::heom_dmma_stage<N, HK, 1, MI, ADJ>;
-    case 2: return heomk::heom_dmma_stage<N, HK, 2, MI, ADJ>;
-    case 4: return heomk::heom_dmma_stage<N, HK, 4, MI, ADJ>;
-    default: return heomk::heom_dmma_stage<N, HK, 8, MI, ADJ>;
+    case 1: return heomk::heom_dmma_stage<N, HK, 1, MI, ADJ, GEN>;
+    case 2: return heomk::heom_dmma_stage<N, HK, 2, MI, ADJ, GEN>;
+    case 4: return heomk::heom_dmma_stage<N, HK, 4, MI, ADJ, GEN>;
+    default: return heomk::heom_dmma_stage<N, HK, 8, MI, ADJ, GEN>;
     }
 }
 
-// variants: one instance, several instances (batch), adjoint of one instance
+// variants: one instance, several instances (batch), adjoint of one instance; the adjoint sweep runs the
+// product form only
 template <int N, int HK>
-dmma_fn_t pick_dmode(int slt, bool multi, bool adj)
+dmma_fn_t pick_dmode(int slt, bool multi, bool adj, bool gen)
 {
-    if (adj) return multi ? pick_dslt<N, HK, true, true>(slt) : pick_dslt<N, HK, false, true>(slt);
-    return multi ? pick_dslt<N, HK, true, false>(slt) : pick_dslt<N, HK, false, false>(slt);
+    if (adj) return multi ? pick_dslt<N, HK, true, true, false>(slt) : pick_dslt<N, HK, false, true, false>(slt);
+    if (gen) return multi ? pick_dslt<N, HK, true, false, true>(slt) : pick_dslt<N, HK, false, false, true>(slt);
+    return multi ? pick_dslt<N, HK, true, false, false>(slt) : pick_dslt<N, HK, false, false, false>(slt);
 }
 
 template <int N>
-dmma_fn_t pick_dn(int hk, int slt, bool multi, bool adj)
+dmma_fn_t pick_dn(int hk, int slt, bool multi, bool adj, bool gen)
 {
-    return hk == heomk::H_REAL_SYM ? pick_dmode<N, heomk::H_REAL_SYM>(slt, multi, adj)
-                                   : pick_dmode<N, heomk::H_GENERIC>(slt, multi, adj);
+    return hk == heomk::H_REAL_SYM ? pick_dmode<N, heomk::H_REAL_SYM>(slt, multi, adj, gen)
+                                   : pick_dmode<N, heomk::H_GENERIC>(slt, multi, adj, gen);
 }
 
 // tensor-pipe kernel: N = 1..8
-dmma_fn_t pick_dmma(int n, int hk, int slt, bool multi, bool adj)
+dmma_fn_t pick_dmma(int n, int hk, int slt, bool multi, bool adj, bool gen)
 {
     switch (n) {
 #define HEOM_CASE(K) \
-    case K: return pick_dn<K>(hk, slt, multi, adj);
+    case K: return pick_dn<K>(hk, slt, multi, adj, gen);
         HEOM_CASE(1) HEOM_CASE(2) HEOM_CASE(3) HEOM_CASE(4) HEOM_CASE(5) HEOM_CASE(6)
         HEOM_CASE(7) HEOM_CASE(8)
 #undef HEOM_CASE
@@ -193,13 +197,13 @@ lock_fn_t pick_lock(int n, int hk, int slt)
 }
 
 // tables that replace the handle's own in one stage launch: those of the
-// adjoint operator L^H (adjoint = true: conj(pf_same_sum), conj(gamma0), -H^H),
-// or those of a time-dependent H(t) (adjoint = false, handle's pss and gamma0)
+// adjoint operator L^H (adjoint = true: conj(gamma0), -H^H), those of a
+// time-dependent H(t) (adjoint = false, handle's gamma0), or a part of L
 struct AdjTabs {
-    const double2* pss;    // conj(pf_same_sum)
     const double2* gamma0; // conj(gamma0)
     const double* hfrag;   // fragments of -H^H
     bool adjoint = true;
+    bool no_same = false;  // leave out pf_same_sum
     // optional bath-coefficient tables (flow tracking: a zero table switches a term off)
     const double* chat = nullptr;
     const double2* khat = nullptr;
@@ -268,9 +272,8 @@ struct heom_handle {
     std::vector<int64_t> top_int; // internal index of each instance's top ADO
 
     // device tables
-    DevBuf<int32_t> d_nbr;
-    DevBuf<uint8_t> d_tup;
-    DevBuf<double2> d_pss, d_hs, d_gamma0;
+    DevBuf<uint8_t> d_rec;           // one record per internal ADO (heomk::PairParams::rec)
+    DevBuf<double2> d_hs, d_gamma0;
     DevBuf<double> d_hfrag;          // per-instance MMA fragments of H / hbar
     DevBuf<int32_t> d_inst;          // instance of each internal ADO (n_inst > 1)
     DevBuf<int64_t> d_top;
@@ -281,7 +284,8 @@ struct heom_handle {
     DevBuf<int64_t> d_int_of_ref, d_ref_of_int;
     DevBuf<int16_t> d_pair;          // [P][2] element indices of the sector halves
     std::vector<int16_t> pair_tab;   // host copy
-    heomk::LaneTab lane_tab{};       // DMMA kernel lane tables (N <= 8)
+    heomk::RowTab row_tab{};         // sector positions of the N <= 8 stage kernel's lanes
+    heomk::LaneTab lane_tab{};       // lane tables of the lockstep kernel
     DevBuf<int> d_err;               // set by a stage kernel whose pipeline wait expired
 
     // propagation state + stage buffers
@@ -295,7 +299,7 @@ struct heom_handle {
 
     // launch accounting and shape
     int64_t launches = 0;
-    int per_sm[2][2] = {{0, 0}, {0, 0}}; // resident stage CTAs per SM, per [adjoint][H kind]
+    int per_sm[3][2] = {{0, 0}, {0, 0}, {0, 0}}; // resident stage CTAs per SM, per [product form, adjoint, any write mode][H kind]
     int grid_override = 0;   // stage grid chosen by an autotuner (0: one full wave)
     size_t stage_smem = 0;
 
@@ -340,54 +344,53 @@ int build_neighbours(heom_handle* h)
     //   plus read only when uid < first_non_plus_id (heom_ode.cl:183) and mask[plus] != 0 (:199)
     //   minus read only when tuple > 0 (:293) and mask[minus] != 0 (:297)
     const int W = h->W, NW = h->NW, TWB = h->TWB;
-    std::vector<int32_t> nbr((size_t)h->nodes * NW, -1);
-    std::vector<uint8_t> tup((size_t)h->nodes * TWB, 0);
-    std::vector<double2> pss(h->nodes);
+    const size_t rb = heomk::rec_bytes(NW, TWB);
+    std::vector<uint8_t> rec((size_t)h->nodes * rb, 0);
     std::vector<int32_t> inst(h->n_inst > 1 ? h->nodes : 0);
     for (int k = 0; k < h->n_inst; ++k) {
         const int64_t base = h->inst_base[k];
         for (int64_t r = base; r < h->inst_base[k + 1]; ++r) {
             const int64_t u = h->int_of_ref[r];
+            uint8_t* row = rec.data() + (size_t)u * rb;
+            int32_t* nbr = reinterpret_cast<int32_t*>(row);
+            uint8_t* tup = row + NW * 4;
+            for (int q = 2 * W; q < NW; ++q) nbr[q] = -1;
             const bool has_plus = r - base < h->inst_fnp[k];
             for (int m = 0; m < W; ++m) {
                 const int32_t t = h->tuples[r * W + m];
-                tup[u * TWB + m] = (uint8_t)t;
+                tup[m] = (uint8_t)t;
                 int32_t pv = -1, mv = -1;
                 const int32_t pr = h->plus[r * W + m];
                 if (has_plus && pr >= 0 && h->mask[pr]) pv = (int32_t)h->int_of_ref[pr];
                 const int32_t mr = h->minus[r * W + m];
                 if (t > 0 && mr >= 0 && h->mask[mr]) mv = (int32_t)h->int_of_ref[mr];
-                nbr[u * NW + 2 * m] = pv;
-                nbr[u * NW + 2 * m + 1] = mv;
+                nbr[2 * m] = pv;
+                nbr[2 * m + 1] = mv;
             }
-            pss[u] = make_double2(h->pss[2 * r], h->pss[2 * r + 1]);
+            std::memcpy(tup + TWB, &h->pss[2 * r], 16);
             if (h->n_inst > 1) inst[u] = k;
         }
     }
-    if (!h->d_nbr.p) {
-        if (int rc = h->d_nbr.alloc(nbr.size())) return rc;
-        if (int rc = h->d_tup.alloc(tup.size())) return rc;
-        if (int rc = h->d_pss.alloc(pss.size())) return rc;
+    if (!h->d_rec.p) {
+        if (int rc = h->d_rec.alloc(rec.size())) return rc;
         if (h->n_inst > 1)
             if (int rc = h->d_inst.alloc(inst.size())) return rc;
     }
-    CUDA_TRY(cudaMemcpy(h->d_nbr.p, nbr.data(), nbr.size() * 4, cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(h->d_tup.p, tup.data(), tup.size(), cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(h->d_pss.p, pss.data(), pss.size() * 16, cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaMemcpy(h->d_rec.p, rec.data(), rec.size(), cudaMemcpyHostToDevice));
     if (h->n_inst > 1) CUDA_TRY(cudaMemcpy(h->d_inst.p, inst.data(), inst.size() * 4, cudaMemcpyHostToDevice));
     return 0;
 }
 
 // device-side forms of one instance's H (interleaved re/im, J): H / hbar
 // row-major (hs) and the MMA operand fragments (frag, heomk::frag_index: lane l = 4g + t, block b, k-slice s,
-// row r = 8b + g, column c = 4s + t; hb = H(c, r), ha = -H(r, c); zero outside N x N)
+// row r = 8b + g, column c = frag_col(N, s, t); hb = H(c, r), ha = -H(r, c); zero outside N x N)
 void h_tables(const double* hk, int N, double2* hs, double* frag)
 {
     for (int q = 0; q < N * N; ++q) hs[q] = make_double2(hk[2 * q] / kHbar, hk[2 * q + 1] / kHbar);
     for (int b = 0; b < heomk::frag_blocks(N); ++b)
         for (int sl = 0; sl < heomk::frag_slices(N); ++sl)
             for (int l = 0; l < 32; ++l) {
-                const int r = 8 * b + (l >> 2), c = 4 * sl + (l & 3);
+                const int r = 8 * b + (l >> 2), c = heomk::frag_col(N, sl, l & 3);
                 if (r >= N || c >= N) continue;
                 const double2 hcr = hs[c * N + r], hrc = hs[r * N + c];
                 frag[heomk::frag_index(N, 0, b, sl, l)] = hcr.x;
@@ -510,9 +513,7 @@ int upload_coefficients(heom_handle* h)
 PairParams base_params(const heom_handle* h)
 {
     PairParams p{};
-    p.nbr = h->d_nbr.p;
-    p.tup = h->d_tup.p;
-    p.pss = h->d_pss.p;
+    p.rec = h->d_rec.p;
     p.hfrag = h->d_hfrag.p;
     p.inst = h->n_inst > 1 ? h->d_inst.p : nullptr;
     p.gamma0 = h->d_gamma0.p;
@@ -552,7 +553,7 @@ int cta_threads(int n) { return (heomk::kCtaWarps / heomk::team_warps(n)) * heom
 int cta_teams(int n) { return heomk::kCtaWarps / heomk::team_warps(n); }
 
 // resolve the launch shape of the stage kernel (outside of any stream capture)
-int resolve_stage(heom_handle* h, const void** fn_out, int* blocks_out = nullptr, bool adj = false)
+int resolve_stage(heom_handle* h, const void** fn_out, int* blocks_out = nullptr, bool adj = false, bool gen = false)
 {
     const void* fn = nullptr;
     size_t smem = 0;
@@ -563,23 +564,23 @@ int resolve_stage(heom_handle* h, const void** fn_out, int* blocks_out = nullptr
         smem = heomk::lockstep_smem_bytes(h->P, h->W, h->NW, h->TWB, h->LS);
         threads = heomk::kLockWarps * 32;
     } else if (h->N <= 8) {
-        fn = (const void*)pick_dmma(h->N, h->hkind, h->SL == 1 ? 1 : h->SLT, h->n_inst > 1, adj); // one slot: exact
+        fn = (const void*)pick_dmma(h->N, h->hkind, h->SL == 1 ? 1 : h->SLT, h->n_inst > 1, adj, gen); // one slot: exact
         smem = heomk::dmma_smem_bytes(h->P, h->W, h->NW, h->TWB, h->LS);
-        threads = heomk::kCtaWarps * 32;
+        threads = heomk::kRowWarps * 32;
     } else {
         fn = (const void*)pick_stage(h->N, h->hkind, h->SL == 1 ? 1 : h->SLT, adj); // one slot: exact
         smem = heomk::pair_smem_bytes(h->N, h->W, h->NW, h->TWB, h->LS);
         threads = cta_threads(h->N);
     }
     if (!fn) return fail(HEOM_E_UNSUPPORTED, "states = %d not supported", h->N);
-    int& per_sm = h->per_sm[adj ? 1 : 0][h->hkind];
+    int& per_sm = h->per_sm[adj ? 1 : gen ? 2 : 0][h->hkind];
     if (per_sm == 0) {
         if (smem > 227 * 1024) return fail(HEOM_E_UNSUPPORTED, "stage kernel needs %zu B of shared memory", smem);
         if (int rc = allow_dynamic_smem(fn, smem)) return rc;
         CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem));
         if (per_sm < 1) return fail(HEOM_E_UNSUPPORTED, "stage kernel cannot be resident");
     }
-    const int teams = h->N <= 8 ? heomk::kCtaWarps : cta_teams(h->N);
+    const int teams = h->N <= 8 ? heomk::kRowWarps : cta_teams(h->N);
     const int64_t groups = h->kp ? h->inst_nodes * (h->kp / 32)
                                  : std::max<int64_t>(1, (h->n_active + teams - 1) / teams);
     const int64_t want = h->grid_override > 0 ? h->grid_override : (int64_t)per_sm * h->sm_count;
@@ -594,16 +595,35 @@ int resolve_stage(heom_handle* h, const void** fn_out, int* blocks_out = nullptr
     return 0;
 }
 
+// launch a stage kernel as a dependent of the kernel before it on the stream: its prologue (tables, lane
+// constants) may run while that one drains; the kernel itself waits before it touches the state
+cudaError_t launch_dependent(const void* fn, int blocks, int threads, size_t smem, cudaStream_t stream, void* params)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    void* args[1] = {params};
+    return cudaLaunchKernelExC(&cfg, fn, args);
+}
+
 int launch_stage(heom_handle* h, int epi, const double2* in, const double2* y, double2* out,
                  double2* acc, double2 beta, int acc_init, const AdjTabs* adj = nullptr,
                  double2 acc_beta = make_double2(0.0, 0.0))
 {
     const void* fn = nullptr;
     int blocks = 0;
-    if (int rc = resolve_stage(h, &fn, &blocks, adj && adj->adjoint)) return rc;
+    if (int rc = resolve_stage(h, &fn, &blocks, adj && adj->adjoint, epi != EPI_AXPY_SELF || (adj && adj->no_same)))
+        return rc;
     PairParams p = base_params(h);
     if (adj) {
-        p.pss = adj->pss;
+        p.no_same = adj->no_same ? 1 : 0;
         p.gamma0 = adj->gamma0;
         p.hfrag = adj->hfrag;
     }
@@ -611,21 +631,20 @@ int launch_stage(heom_handle* h, int epi, const double2* in, const double2* y, d
     p.out = out;
     switch (epi) {
     case EPI_PURE:
-        p.alpha = make_double2(0.0, 0.0);
         p.beta = make_double2(1.0, 0.0);
         break;
     case EPI_AXPY_SELF:
-        p.alpha = make_double2(1.0, 0.0);
+        p.use_x = 1;
         p.beta = beta;
         break;
     case EPI_AXPY_Y:
         p.y = y;
-        p.alpha = make_double2(1.0, 0.0);
+        p.use_x = 1;
         p.beta = beta;
         break;
     case EPI_AXPY_ACC:
         p.y = y;
-        p.alpha = make_double2(1.0, 0.0);
+        p.use_x = 1;
         p.beta = beta;
         p.acc = acc;
         p.use_acc = 1;
@@ -633,7 +652,6 @@ int launch_stage(heom_handle* h, int epi, const double2* in, const double2* y, d
         p.acc_init = acc_init;
         break;
     default: // EPI_ACC
-        p.alpha = make_double2(0.0, 0.0);
         p.beta = make_double2(1.0, 0.0);
         p.acc = acc;
         p.use_acc = 1;
@@ -643,7 +661,7 @@ int launch_stage(heom_handle* h, int epi, const double2* in, const double2* y, d
     }
     heomk::DmmaParams dp;
     dp.p = p;
-    dp.lt = h->lane_tab;
+    dp.rt = h->row_tab;
     dp.ct.chat = adj && adj->chat ? adj->chat : h->d_chat.p;
     dp.ct.khat = adj && adj->khat ? adj->khat : h->d_khat.p;
     dp.ct.sq = h->d_sq.p;
@@ -655,19 +673,18 @@ int launch_stage(heom_handle* h, int epi, const double2* in, const double2* y, d
         lp.p = dp.p;
         lp.p.nodes = h->inst_nodes;
         lp.p.inst = nullptr;
-        lp.lt = dp.lt;
+        lp.lt = h->lane_tab;
         lp.ct = dp.ct;
         lp.K = h->n_inst;
         lp.Kp = (int)h->kp;
         lp.nodes = h->inst_nodes;
-        ((lock_fn_t)fn)<<<blocks, heomk::kLockWarps * 32, h->stage_smem, h->stream>>>(lp);
+        CUDA_TRY(launch_dependent(fn, blocks, heomk::kLockWarps * 32, h->stage_smem, h->stream, &lp));
         h->launches++;
-        CUDA_TRY(cudaGetLastError());
         return 0;
     }
-    ((dmma_fn_t)fn)<<<blocks, h->N <= 8 ? heomk::kCtaWarps * 32 : cta_threads(h->N), h->stage_smem, h->stream>>>(dp);
+    CUDA_TRY(launch_dependent(fn, blocks, h->N <= 8 ? heomk::kRowWarps * 32 : cta_threads(h->N), h->stage_smem,
+                              h->stream, &dp));
     h->launches++;
-    CUDA_TRY(cudaGetLastError());
     return 0;
 }
 
@@ -704,7 +721,7 @@ int launch_flows(heom_handle* h, const double2* in, double acc_coeff)
         heom_buffer* dst = part == 0 ? h->flow_above : h->flow_below;
         if (!dst) continue;
         AdjTabs t;
-        t.pss = z2;
+        t.no_same = true;
         t.gamma0 = z2;
         t.hfrag = z1;
         t.adjoint = false;
@@ -750,7 +767,6 @@ heomk::FieldParams field_params(heom_handle* h, int nt)
 AdjTabs field_tabs(const heom_handle* h, int s)
 {
     AdjTabs t;
-    t.pss = h->d_pss.p;
     t.gamma0 = h->d_gamma0.p;
     t.hfrag = h->field_frag.p + (size_t)s * h->n_inst * heomk::frag_doubles(h->N);
     t.adjoint = false;
@@ -982,17 +998,17 @@ int check_same_class(const heom_instance_desc* a, const heom_instance_desc* b)
     return 0;
 }
 
-// sector tables of the pair layout: the searched order for N <= 8
-// (pair_tables.inc), the canonical order of heomk::pair_elements above
-int build_pair_tables(heom_handle* h)
+// sector tables of the pair layout: the searched orders for N <= 8 (row_tables.inc; pair_tables.inc for the
+// lockstep layout), the canonical order of heomk::pair_elements above
+int build_pair_tables(heom_handle* h, bool lockstep = false)
 {
     const int N = h->N, P = h->P;
     h->pair_tab.assign(2 * P, 0);
     for (int p = 0; p < P; ++p) {
         int e1, e2, i, j, d;
         if (N <= 8) {
-            e1 = kPairE1[N][p];
-            e2 = kPairE2[N][p];
+            e1 = lockstep ? kPairE1[N][p] : kRowE1[N][p];
+            e2 = lockstep ? kPairE2[N][p] : kRowE2[N][p];
         } else {
             heomk::pair_elements(N, p, &e1, &e2, &i, &j, &d);
         }
@@ -1006,17 +1022,31 @@ int build_pair_tables(heom_handle* h)
             lt.e2[l] = (signed char)(l < P ? h->pair_tab[2 * l + 1] : 0);
             const int r = l >> 2, t = l & 3;
             for (int s = 0; s < 2; ++s) {
-                const int k = 4 * s + t;
+                const int k = 2 * t + s;
                 lt.fs[l][s] = -1;
                 lt.ha[l][s] = 0;
-                if (r >= N || k >= N) continue;
-                const int e = r * N + k;
-                for (int p = 0; p < P; ++p) {
-                    if (h->pair_tab[2 * p] == e) { lt.fs[l][s] = (signed char)p; lt.ha[l][s] = 0; break; }
-                    if (h->pair_tab[2 * p + 1] == e) { lt.fs[l][s] = (signed char)p; lt.ha[l][s] = 1; break; }
+                if (r < N && k < N) {
+                    const int e = r * N + k;
+                    for (int p = 0; p < P && lt.fs[l][s] < 0; ++p)
+                        for (int hf = 0; hf < 2 && lt.fs[l][s] < 0; ++hf)
+                            if (h->pair_tab[2 * p + hf] == e) {
+                                lt.fs[l][s] = (signed char)p;
+                                lt.ha[l][s] = (signed char)hf;
+                            }
+                    if (lt.fs[l][s] < 0) return fail(HEOM_E_UNSUPPORTED, "pair table misses element %d", e);
                 }
-                if (lt.fs[l][s] < 0) return fail(HEOM_E_UNSUPPORTED, "pair table misses element %d", e);
+                h->row_tab.pos[l][s] = lt.fs[l][s];
             }
+        }
+        // the diagonal sectors, whose bath terms are half of the others', all go to the first warp of the lockstep
+        // kernel: it takes one sector more than the rest (N = 7: 4 of 25, the others 3)
+        std::vector<int> diag, off;
+        for (int p = 0; p < P; ++p)
+            (h->pair_tab[2 * p] % (N + 1) == 0 ? diag : off).push_back(p);
+        size_t nd = 0, no = 0;
+        for (int k = 0; k < P; ++k) {
+            const bool d = no == off.size() || (k % heomk::kLockWarps == 0 && nd < diag.size());
+            lt.ord[k] = (signed char)(d ? diag[nd++] : off[no++]);
         }
     }
     if (int rc = h->d_pair.alloc(2 * P)) return rc;
@@ -1145,10 +1175,17 @@ int make_lockstep(heom_handle* h)
     if (cudaMalloc(&ny, elems * sizeof(double2)) != cudaSuccess)
         return fail(HEOM_E_NOMEM, "lockstep layout: cudaMalloc of %zu bytes failed", elems * sizeof(double2));
     const std::vector<int64_t> tops(h->n_inst, h->top_int[0] - h->inst_base[0]);
+    if (int rc = build_pair_tables(h, true)) {
+        build_pair_tables(h);
+        cudaFree(ny);
+        return rc;
+    }
     if (cudaMemset(ny, 0, elems * sizeof(double2)) != cudaSuccess ||
         cudaMemcpy(h->d_top.p, tops.data(), tops.size() * 8, cudaMemcpyHostToDevice) != cudaSuccess) {
+        const cudaError_t err = cudaGetLastError();
+        build_pair_tables(h);
         cudaFree(ny);
-        return fail(HEOM_E_CUDA, "lockstep layout: %s", cudaGetErrorString(cudaGetLastError()));
+        return fail(HEOM_E_CUDA, "lockstep layout: %s", cudaGetErrorString(err));
     }
     h->y.data.reset();
     h->y.data.p = ny;
@@ -2577,7 +2614,7 @@ void* heom_ensemble_stream(heom_ensemble* e) { return e ? (void*)e->stream : nul
 struct heom_adjoint {
     heom_handle* h = nullptr;
     AdjTabs tabs{};
-    DevBuf<double2> pss_adj, g0_adj;
+    DevBuf<double2> g0_adj;
     DevBuf<double> hfrag_adj;
     DevBuf<double> dpss;       // [nodes] d pf_same_sum / d gamma (internal order)
     DevBuf<double2> dg0;       // [2][N*N]
@@ -2624,10 +2661,7 @@ int adj_tables(heom_adjoint* A, const heomhost::system_params& sp)
 {
     heom_handle* h = A->h;
     const int N = h->N, W = h->W, M = h->M, K = h->n_inst;
-    // L^H: conj(pf_same_sum), conj(gamma0), -H^H
-    std::vector<double2> pss(h->nodes);
-    for (int64_t r = 0; r < h->nodes; ++r)
-        pss[h->int_of_ref[r]] = make_double2(h->pss[2 * r], -h->pss[2 * r + 1]);
+    // L^H: conj(gamma0), -H^H (the kernel conjugates pf_same_sum)
     std::vector<double2> g0 = gamma0_table(h, h->pf_same);
     for (auto& v : g0) v.y = -v.y;
     std::vector<double2> hs((size_t)N * N);
@@ -2642,13 +2676,11 @@ int adj_tables(heom_adjoint* A, const heomhost::system_params& sp)
             }
         h_tables(hadj.data(), N, hs.data(), frag.data() + (size_t)k * fd);
     }
-    if (int rc = A->pss_adj.alloc(pss.size())) return rc;
     if (int rc = A->g0_adj.alloc(g0.size())) return rc;
     if (int rc = A->hfrag_adj.alloc(frag.size())) return rc;
-    CUDA_TRY(cudaMemcpy(A->pss_adj.p, pss.data(), pss.size() * 16, cudaMemcpyHostToDevice));
     CUDA_TRY(cudaMemcpy(A->g0_adj.p, g0.data(), g0.size() * 16, cudaMemcpyHostToDevice));
     CUDA_TRY(cudaMemcpy(A->hfrag_adj.p, frag.data(), frag.size() * 8, cudaMemcpyHostToDevice));
-    A->tabs = AdjTabs{A->pss_adj.p, A->g0_adj.p, A->hfrag_adj.p};
+    A->tabs = AdjTabs{A->g0_adj.p, A->hfrag_adj.p};
 
     // derivative tables for theta = lambda (0), gamma (1)
     heomhost::bath_derivs bd = heomhost::bath_derivatives(sp);
@@ -2696,8 +2728,7 @@ int adj_grad(heom_adjoint* A, const double2* a, const double2* w, double2 weight
     heomk::GradParams g{};
     g.a = a;
     g.w = w;
-    g.nbr = h->d_nbr.p;
-    g.tup = h->d_tup.p;
+    g.rec = h->d_rec.p;
     g.pe = h->d_pair.p;
     g.slots = h->d_slots.p;
     g.dpss = A->dpss.p;
