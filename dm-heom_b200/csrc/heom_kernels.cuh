@@ -46,7 +46,9 @@ constexpr int kCtaWarps = 8;
 constexpr int kRowWarps = 4; // warps of a CTA of the N <= 8 stage kernel
 
 __host__ __device__ constexpr int pairs_of(int n) { return n * (n - 1) / 2 + (n + 1) / 2; }
-__host__ __device__ constexpr int team_warps(int n) { return (pairs_of(n) + 31) / 32; }
+__host__ __device__ constexpr int team_warps(int n) { return (n * ((n + 1) / 2) + 31) / 32; }
+__host__ __device__ constexpr int cta_teams(int n) { return team_warps(n) == 2 ? 2 : 1; }
+__host__ __device__ constexpr int team_threads(int n) { return cta_teams(n) * team_warps(n) * 32; }
 
 // element indices (row-major, e = i*N + j) of the two halves of sector p
 __host__ __device__ inline void pair_elements(int n, int p, int* e1, int* e2, int* i_out, int* j_out,
@@ -139,9 +141,10 @@ __host__ __device__ inline int dmma_lut_bytes(int W, int LS)
 // dynamic shared memory carve-up (bytes); everything 16-B aligned
 struct PairSmem {
     int lut;     // coefficient tables (dmma_lut_bytes)
-    int team;    // per team: 2 slots + the exchange tile
+    int team;    // per team: 2 slots, 2 exchange tiles, the hand-over buffers, gamma0
     int slot;    // per slot: tile + nbr + tup + pss
     int tile_off, nbr_off, tup_off, pss_off, xch_off;
+    int hand_off, gam_off; // terms handed over (two copies of [2][threads]), gamma0 of the owned elements
 };
 
 __host__ __device__ inline PairSmem pair_smem_layout(int n, int W, int NW, int TWB, int LS)
@@ -155,15 +158,16 @@ __host__ __device__ inline PairSmem pair_smem_layout(int n, int W, int NW, int T
     s.pss_off = s.tup_off + ((TWB + 15) & ~15);
     s.slot = s.pss_off + 16;
     s.xch_off = 2 * s.slot;
-    s.team = s.xch_off + kXchBytes;
+    s.hand_off = s.xch_off + 2 * kXchBytes;
+    s.gam_off = s.hand_off + 2 * 2 * team_warps(n) * 32 * 16;
+    s.team = s.gam_off + 2 * team_warps(n) * 32 * 16;
     return s;
 }
 
 __host__ inline size_t pair_smem_bytes(int n, int W, int NW, int TWB, int LS)
 {
     const PairSmem s = pair_smem_layout(n, W, NW, TWB, LS);
-    const int teams = kCtaWarps / team_warps(n);
-    return (size_t)s.lut + (size_t)teams * s.team;
+    return (size_t)s.lut + (size_t)cta_teams(n) * s.team;
 }
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem)
@@ -773,121 +777,179 @@ __global__ void __launch_bounds__(kRowWarps * 32, row_blocks(HK, SLT, MI)) heom_
 // ---------------------------------------------------------------------------
 
 // ---------------------------------------------------------------------------
-// N = 9..16: a team of TW = ceil(P / 32) warps per ADO, thread p of the team
-// owns sector p.  Teams loop over ADOs (grid-stride) with a two-slot
-// pipeline: while ADO k is computed, its successor's tile (scattered into the
-// row-major tile_pos layout), neighbour row, tuple row and pf_same_sum arrive
-// by cp.async.
+// N = 9..16: a team of TW warps per ADO, one thread per (state r, column pair
+// t): thread r T + t of the team, T = ceil(N / 2), works as lane (r, t) of
+// heom_dmma_stage does: it reads its two sectors {r, 2t}, {r, 2t+1} of the
+// neighbours along the baths of state r, writes the sector it owns and hands
+// the terms of the other one over to its owner.  The sectors are numbered in
+// the order of their owners' threads.
 //
 // Commutator on the FP64 tensor pipe: the tile is zero-padded to 16 x 16 and
 // cut into 2 x 2 blocks of 8 x 8; block (I, J) of C = w H - H w takes
 // ceil(N/4) k-slices of m8n8k4 MMAs (A = w(8I+g, 4s+t) against the H
 // fragment hb(J, s); ha(I, s) against B = w(4s+t, 8J+g)).  Warp wt of the
 // team computes blocks [4 wt / TW, 4 (wt+1) / TW) and writes them to the
-// team's exchange tile; after a team barrier every owner reads the two
-// elements of its sector.  (Cutting the work finer, into the real and
-// imaginary parts of each block, balances the warps of a three-warp team but
-// doubles the operand reads and measured slower.)  The bath terms follow the
-// same formulas as the DMMA kernel, one 32-byte sector load per neighbour.
+// team's exchange tile.
+//
+// Per ADO the team meets once: before the barrier every warp writes its blocks
+// and its handed-over terms, and waits for its copies of the next ADO (two
+// slots, cp.async); after it, the owners read the commutator and the terms
+// handed to them, and the neighbours of the next ADO are asked for.  The
+// exchange tile and the hand-over buffer alternate between two copies, so
+// that no second barrier is needed.
+//
+// What bounds it: 18 to 20 warps per SM (96 registers) with the L1 data pipe
+// 69 % busy (12 states, two slots: 512 wavefronts of 747 cycles per ADO and SM,
+// 373 of them shared memory) and the FP64 tensor pipe a quarter.  Measured
+// against a thread per sector with two barriers per ADO (us per stage, one
+// B200): 12 states, two slots, 20,475 ADOs 74.5 -> 55.5 (24 warps of 80
+// registers: 66), one slot, 18,564 ADOs 51.9 -> 43.1; 10 states, two slots,
+// 10,626 ADOs 29.4 -> 24.4; 9 states, one slot, 5005 ADOs 13.9 -> 11.8; 11
+// states (three warps instead of two), one slot, 12,376 ADOs 29.3 -> 28.6.
 // ---------------------------------------------------------------------------
 
-// issue the asynchronous copies of ADO u into a team slot
-template <int N>
-__device__ __forceinline__ void prefetch_ado(unsigned char* slot, const PairParams& p, const PairSmem& L,
-                                             int64_t u, int lt, int tt, int e1, int e2, bool active)
+// position of the sector owned by thread (r, t): threads of odd rows own
+// nothing in the last column pair of an odd N
+__host__ __device__ constexpr int team_pos(int n, int r, int t) { return r * ((n + 1) / 2) + t - ((n & 1) ? r >> 1 : 0); }
+
+// CTAs per SM: 96 registers a thread where that does not spill (five warps on each SM partition), else 128 (four)
+constexpr int team_blocks(int n, int hk, int slt)
 {
-    double2* tile = reinterpret_cast<double2*>(slot + L.tile_off);
-    if (active) {
-        const double2* src = p.in + u * (2 * pairs_of(N));
-        const int i1 = e1 / N, j1 = e1 - i1 * N, i2 = e2 / N, j2 = e2 - i2 * N;
-        cp_async16(tile + tile_pos(N, i1, j1), src + 2 * lt);
-        cp_async16(tile + tile_pos(N, i2, j2), src + 2 * lt + 1);
-    }
-    // the record's parts lie back to back in the slot
-    const int recb = rec_bytes(p.NW, p.TWB);
-    for (int q = lt * 16; q < recb; q += tt * 16) cp_async16(slot + L.nbr_off + q, p.rec + u * recb + q);
+    const bool small = hk == H_REAL_SYM && slt <= 2;
+    return team_warps(n) == 3 ? (small ? 6 : 5) : (small ? 5 : 4);
 }
 
-// ADJ: the adjoint operator L^H (see heom_dmma_stage).  The bath
-// coefficients are the factored tables of heom_dmma_stage (CoefTabs).
-// (three CTAs per SM where at most two slots per state keep the register
-// demand low enough; two otherwise)
+// ADJ: the adjoint operator L^H (see heom_dmma_stage, also for K and C).  The
+// bath coefficients are the factored tables of heom_dmma_stage (CoefTabs).
 template <int N, int HK, int SLT, bool ADJ>
-__global__ void __launch_bounds__(kCtaWarps * 32, SLT <= 2 ? 3 : 2) heom_pair_stage(const __grid_constant__ DmmaParams dp)
+__global__ void __launch_bounds__(team_threads(N), team_blocks(N, HK, SLT))
+    heom_pair_stage(const __grid_constant__ DmmaParams dp)
 {
     static_assert(N > 8 && N <= 16, "team kernel handles N = 9..16");
     constexpr int P = pairs_of(N);
+    constexpr int T = (N + 1) / 2;
     constexpr int TW = team_warps(N);
     constexpr int TT = 32 * TW;
-    constexpr int TEAMS = kCtaWarps / TW;
     constexpr int KS = (N + 3) / 4; // k-slices of the padded commutator
     constexpr int FD = frag_doubles(N);
+    constexpr int QB = SLT < 2 ? SLT : 2; // slots whose neighbours are read in one batch
+    constexpr bool ODD = (N & 1) != 0;
     extern __shared__ __align__(128) unsigned char smem[];
     const PairParams& p = dp.p;
     const PairSmem L = pair_smem_layout(N, p.W, p.NW, p.TWB, p.LS);
     const int W = p.W, LS = p.LS, SL = p.SL;
-    grid_launch_dependents();
 
-    double2* s_kh = reinterpret_cast<double2*>(smem);      // 3 * W
+    grid_launch_dependents();
+    double2* s_kh = reinterpret_cast<double2*>(smem);      // [3][W]: kappa_i, kappa_j, kappa_i + kappa_j
     double2* s_sq = s_kh + 3 * W;                           // LS + 1: (sqrt(n), sqrt(n+1))
     double* s_ch = reinterpret_cast<double*>(s_sq + LS + 1); // W
-    int16_t* s_pos = reinterpret_cast<int16_t*>(s_ch + W);   // W
     for (int q = threadIdx.x; q < 3 * W; q += blockDim.x) s_kh[q] = dp.ct.khat[q];
     for (int q = threadIdx.x; q < W; q += blockDim.x) s_ch[q] = dp.ct.chat[q];
     for (int q = threadIdx.x; q <= LS; q += blockDim.x)
         s_sq[q] = make_double2(dp.ct.sq[q], q < LS ? dp.ct.sq[q + 1] : 0.0);
-    for (int q = threadIdx.x; q < W; q += blockDim.x) s_pos[q] = dp.ct.pos[q];
 
     const int team = threadIdx.x / TT;
     const int lt = threadIdx.x - team * TT;
-    const bool active = team < TEAMS && lt < P;
     unsigned char* team_base = smem + L.lut + team * L.team;
-    double2* xch = reinterpret_cast<double2*>(team_base + L.xch_off);
     const int wt = lt >> 5, lane = lt & 31, g = lane >> 2, t4 = lane & 3;
     const int blk0 = wt * 4 / TW, blk1 = (wt + 1) * 4 / TW; // commutator blocks of this warp
+    // operand and result positions of block (0, 0) and slice 0 (tile_pos: the swap of columns k ^ (i & 2) leaves
+    // multiples of four alone, so that blocks and slices add constants)
+    constexpr int TS = tile_stride(N);
+    const int oa = g * TS + (t4 ^ (g & 2)), ob = t4 * TS + (g ^ (t4 & 2)), xw = g * kXchStride + 2 * t4;
 
-    int e1 = 0, e2 = 0, i = 0, j = 0, diag = 0;
-    if (active) pair_elements(N, lt, &e1, &e2, &i, &j, &diag);
+    // ---- this thread's place ----
+    const bool active = lt < N * T;
+    const int r = active ? lt / T : 0, t = active ? lt - r * T : 0, R = r >> 1;
+    const int odd = row_owned(r, t);                        // owns {r, 2t + odd}
+    const int co = 2 * t + odd, cg = 2 * t + 1 - odd;       // columns owned, handed over
+    const bool dga = t == R && !(r & 1), dgb = t == R && (r & 1); // the diagonal sector is owned / handed over
+    const bool owner = active && co < N, holds = active && cg < N;
+    const int ro = t == R ? r ^ 1 : cg, tr = t == R ? t : R; // row and column pair of the thread that owns it
+    const int pso = team_pos(N, r, t), psg = team_pos(N, ro, tr), rid = ro * T + tr;
+    const int i2 = dga ? (r + 1 < N ? r + 1 : r) : co, j2 = dga ? i2 : r; // second element of the owned sector
+    const int tp1 = owner ? tile_pos(N, r, co) : 0, tp2 = owner ? tile_pos(N, i2, j2) : 0;
+    const int xc1 = r * kXchStride + co, xc2 = i2 * kXchStride + j2;
+    // negative: no such sector; no C term on it (diagonal)
+    const int no_o = owner ? 0 : -1, no_g = holds ? 0 : -1;
+    const int no_co = dga ? -1 : no_o, no_cg = dgb ? -1 : no_g;
+    const double2* in_o = p.in + 2 * (owner ? pso : 0);
+    const double2* in_g = p.in + 2 * (holds ? psg : 0);
 
-    const double2 g1 = active ? p.gamma0[e1] : make_double2(0.0, 0.0);
-    const double2 g2 = active ? p.gamma0[e2] : make_double2(0.0, 0.0);
-    int sli[SLT], slj[SLT];
+    int slo[SLT], kp[SLT]; // slots of state r and their table positions (-1: none)
 #pragma unroll
     for (int q = 0; q < SLT; ++q) {
-        sli[q] = (active && q < SL) ? p.slots[i * SL + q] : -1;
-        slj[q] = (active && q < SL) ? p.slots[j * SL + q] : -1;
+        const int sl = (active && q < SL) ? p.slots[r * SL + q] : -1;
+        slo[q] = sl >= 0 ? sl : 0;
+        kp[q] = sl >= 0 ? dp.ct.pos[sl] : -1;
     }
-    // coefficient tables seen by the two elements of this sector
-    const double2* kap_i1 = s_kh + (diag ? 2 : 0) * W; // element 1, slots of site i
-    const double2* kap_j1 = s_kh + 1 * W;              // element 1, slots of site j (off-diagonal)
-    const double2* kap_i2 = s_kh + 1 * W;              // element 2 = (j,i), slots of site i (its j side)
-    const double2* kap_j2 = s_kh + (diag ? 2 : 0) * W; // element 2, slots of site j
-
+    const double2* kt_of = s_kh + (dga ? 2 : 0) * W;
+    const double2* kt_gs = s_kh + (dgb ? 2 : 0) * W;
+    const double2* kt_j = s_kh + W;
+    double2* s_gam = reinterpret_cast<double2*>(team_base + L.gam_off); // [2][TT]: gamma0 of the owned elements
+    s_gam[lt] = owner ? p.gamma0[r * N + co] : make_double2(0.0, 0.0);
+    s_gam[TT + lt] = owner ? p.gamma0[i2 * N + j2] : make_double2(0.0, 0.0);
+    // terms handed over, two copies of [2][TT]; what nobody hands over (the last diagonal element of an odd N) stays zero
+    double2* hand = reinterpret_cast<double2*>(team_base + L.hand_off);
+    for (int q = 0; q < 4; ++q) hand[q * TT + lt] = make_double2(0.0, 0.0);
     __syncthreads();
-    if (team >= TEAMS) return;
     grid_wait(); // the state and the H tables of a field are written by the kernels before this one
 
-    const int64_t nodes = p.nodes;
-    const int64_t stride = (int64_t)gridDim.x * TEAMS;
-    int64_t u = (int64_t)blockIdx.x * TEAMS + team;
-    int cur = 0;
-    if (u < nodes) prefetch_ado<N>(team_base, p, L, u, lt, TT, e1, e2, active);
+    const unsigned nodes = (unsigned)p.nodes; // at most 2^31 - 1
+    constexpr int TEAMS = cta_teams(N);
+    const unsigned stride = gridDim.x * TEAMS;
+    unsigned u = blockIdx.x * TEAMS + team;
+    const int recb = rec_bytes(p.NW, p.TWB);
+
+    // issue the asynchronous copies of ADO v into a slot: its own sector by every owner (scattered into the
+    // row-major tile), the record by the first threads
+    auto prefetch = [&](unsigned v, unsigned char* slot) {
+        double2* tile = reinterpret_cast<double2*>(slot + L.tile_off);
+        if (owner) {
+            const double2* src = in_o + (int64_t)v * (2 * P);
+            cp_async16(tile + tp1, src);
+            cp_async16(tile + tp2, src + 1);
+        }
+        for (int q = lt * 16; q < recb; q += TT * 16) cp_async16(slot + L.nbr_off + q, p.rec + (int64_t)v * recb + q);
+    };
+    // the neighbours of the first slots' batch (QB slots) are read one ADO ahead: vk, vc their indices along K and C,
+    // xo, xg the K neighbours' sectors
+    int vk[QB], vc[QB];
+    double2 xo[QB][2], xg[QB][2];
+    auto load_k = [&](const unsigned char* slot, int q0) {
+        const int2* nb = reinterpret_cast<const int2*>(slot + L.nbr_off);
+#pragma unroll
+        for (int b = 0; b < QB; ++b) {
+            const int2 pm = kp[q0 + b] >= 0 ? nb[slo[q0 + b]] : make_int2(-1, -1);
+            vk[b] = ADJ ? pm.x : pm.y;
+            vc[b] = ADJ ? pm.y : pm.x;
+            const int64_t o = (int64_t)vk[b] * (2 * P);
+            ld256_if(ODD ? vk[b] | no_o : vk[b], in_o + o, xo[b][0], xo[b][1]);
+            ld256_if(ODD ? vk[b] | no_g : vk[b], in_g + o, xg[b][0], xg[b][1]);
+        }
+    };
+
+    unsigned it = 0;
+    if (u < nodes) prefetch(u, team_base);
     cp_async_wait_all();
     team_sync<TW>(team);
-    int ci = (p.inst && u < nodes) ? __ldg(p.inst + u) : 0; // instance of the current ADO
-
-    for (; u < nodes; u += stride) {
-        unsigned char* slot = team_base + cur * L.slot;
-        const int64_t un = u + stride;
-        int ni = ci;
-        if (un < nodes) {
-            prefetch_ado<N>(team_base + (cur ^ 1) * L.slot, p, L, un, lt, TT, e1, e2, active);
-            if (p.inst) ni = __ldg(p.inst + un);
-        }
-        const double2* t = reinterpret_cast<const double2*>(slot + L.tile_off);
+    if (u < nodes) load_k(team_base, 0);
+    for (; u < nodes; u += stride, ++it) {
+        const unsigned char* slot = team_base + (it & 1) * L.slot;
+        unsigned char* slot_n = team_base + ((it & 1) ^ 1) * L.slot;
+        const bool more = u + stride < nodes;
+        if (more) prefetch(u + stride, slot_n); // its last readers are behind the barrier of the previous iteration
+        const double2* tile = reinterpret_cast<const double2*>(slot + L.tile_off);
+        const unsigned char* tu = slot + L.tup_off;
+        double2* xch = reinterpret_cast<double2*>(team_base + L.xch_off + (it & 1) * kXchBytes);
+        double2* hnd = hand + (it & 1) * 2 * TT;
 
         // ---- commutator w H - H w / hbar on the tensor pipe, into the exchange tile ----
-        const double* fr = p.hfrag + (size_t)ci * FD;
+        // (rows and columns of an operand outside N x N are not read from the result and may hold anything; a
+        // contraction index outside must be zero)
+        const double* fr = p.hfrag + (p.inst ? (size_t)__ldg(p.inst + u) * FD : 0) + lane;
+        const double2* ta = tile + oa;
+        const double2* tb = tile + ob;
 #pragma unroll
         for (int blk = 0; blk < 4; ++blk) {
             if (blk < blk0 || blk >= blk1) continue;
@@ -895,147 +957,128 @@ __global__ void __launch_bounds__(kCtaWarps * 32, SLT <= 2 ? 3 : 2) heom_pair_st
             double cr0 = 0.0, cr1 = 0.0, ci0 = 0.0, ci1 = 0.0;
 #pragma unroll
             for (int s = 0; s < KS; ++s) {
-                const int ra = 8 * I + g, ka = 4 * s + t4; // A = w(ra, ka), B = w(ka, cb)
-                const int cb = 8 * J + g;
+                // A = w(8I+g, 4s+t4), B = w(4s+t4, 8J+g)
+                const bool in = 4 * s + 3 < N || 4 * s + t4 < N;
                 const double2 z = make_double2(0.0, 0.0);
-                const double2 A = (ra < N && ka < N) ? t[tile_pos(N, ra, ka)] : z;
-                const double2 B = (ka < N && cb < N) ? t[tile_pos(N, ka, cb)] : z;
-                const double hbr = fr[frag_index(N, 0, J, s, lane)];
-                const double har = fr[frag_index(N, 2, I, s, lane)];
+                const double2 A = in ? ta[8 * I * TS + 4 * s] : z;
+                const double2 B = in ? tb[8 * J + 4 * s * TS] : z;
+                const double hbr = fr[frag_index(N, 0, J, s, 0)];
                 dmma(cr0, cr1, A.x, hbr); // Re(w) Re(H)
                 dmma(ci0, ci1, A.y, hbr); // Im(w) Re(H)
-                dmma(cr0, cr1, har, B.x); // -Re(H) Re(w)
-                dmma(ci0, ci1, har, B.y); // -Re(H) Im(w)
                 if (HK == H_GENERIC) {
-                    const double hbi = fr[frag_index(N, 1, J, s, lane)];
-                    const double hai = fr[frag_index(N, 3, I, s, lane)];
+                    const double har = fr[frag_index(N, 2, I, s, 0)];
+                    const double hbi = fr[frag_index(N, 1, J, s, 0)];
+                    const double hai = fr[frag_index(N, 3, I, s, 0)];
+                    dmma(cr0, cr1, har, B.x);  // -Re(H) Re(w)
+                    dmma(ci0, ci1, har, B.y);  // -Re(H) Im(w)
                     dmma(cr0, cr1, -A.y, hbi); // -Im(w) Im(H)
                     dmma(ci0, ci1, A.x, hbi);  //  Re(w) Im(H)
                     dmma(cr0, cr1, -hai, B.y); // +Im(H) Im(w)
                     dmma(ci0, ci1, hai, B.x);  // -Im(H) Re(w)
+                } else { // H(r, k) = H(k, r): block I's fragment of w H is that of H w with the sign changed
+                    const double hir = I == J ? hbr : fr[frag_index(N, 0, I, s, 0)];
+                    dmma(cr0, cr1, hir, -B.x);
+                    dmma(ci0, ci1, hir, -B.y);
                 }
             }
-            double2* xr = xch + (8 * I + g) * kXchStride + 8 * J + 2 * t4;
+            double2* xr = xch + xw + 8 * I * kXchStride + 8 * J;
             xr[0] = make_double2(cr0, ci0);
             xr[1] = make_double2(cr1, ci1);
         }
 
-        // the bath terms first: they need only the staged tile and the
-        // neighbours, so a warp that finished its commutator blocks goes on
-        // while the others complete theirs; the exchange tile is read after
-        // the team barrier
-        const int i1 = e1 / N, j1 = e1 - i1 * N, i2 = e2 / N, j2 = e2 - i2 * N;
-        double2 L1 = make_double2(0.0, 0.0), L2 = L1, s1 = L1, s2 = L1;
-        if (active) {
-            const int32_t* nb = reinterpret_cast<const int32_t*>(slot + L.nbr_off);
-            const unsigned char* tu = slot + L.tup_off;
-            double2 pss = *reinterpret_cast<const double2*>(slot + L.pss_off);
-            if (p.no_same) pss = make_double2(0.0, 0.0);
-            if (ADJ) pss.y = -pss.y;
-            s1 = t[tile_pos(N, i1, j1)];
-            s2 = t[tile_pos(N, i2, j2)];
-
-            // ---- same term ----
-            cmac(L1, make_double2(pss.x + g1.x, pss.y + g1.y), s1);
-            cmac(L2, make_double2(pss.x + g2.x, pss.y + g2.y), s2);
-
-            // ---- neighbours: per side all loads first, then the updates ----
-            // side 0 = slots of site i, side 1 = slots of site j
-            // one slot per state: both sides' neighbour rows in one batch
-            constexpr int SB = SLT == 1 ? 2 : 1;
+        // ---- same term of the owned elements ----
+        double2 pss = *reinterpret_cast<const double2*>(slot + L.pss_off);
+        if (p.no_same) pss = make_double2(0.0, 0.0);
+        if (ADJ) pss.y = -pss.y;
+        const double2 xf = tile[tp1], xs = tile[tp2];
+        double2 of = make_double2(0.0, 0.0), os = of, gf = of, gs = of; // owned / handed-over sector, first / second half
+        {
+            const double2 g1 = s_gam[lt], g2 = s_gam[TT + lt];
+            cmac(of, make_double2(pss.x + g1.x, pss.y + g1.y), xf);
+            cmac(os, make_double2(pss.x + g2.x, pss.y + g2.y), xs);
+        }
 #pragma unroll
-            for (int sd0 = 0; sd0 < 2; sd0 += SB) {
-                double2 xp[SB][SLT][2], xm[SB][SLT][2];
-                int nn[SB][SLT];
+        for (int q0 = 0; q0 < SLT; q0 += QB) {
+            if (q0 > 0) load_k(slot, q0);
+            // ---- bath terms: K neighbours ----
 #pragma unroll
-                for (int bb = 0; bb < SB; ++bb) {
-                    const int sd = sd0 + bb;
-#pragma unroll
-                    for (int q = 0; q < SLT; ++q) {
-                        const int sl = sd == 0 ? sli[q] : slj[q];
-                        const int2 pm = sl >= 0 ? reinterpret_cast<const int2*>(nb)[sl] : make_int2(-1, -1);
-                        const int32_t vp = (ADJ || !diag) ? pm.x : -1;
-                        const int32_t vm = (!ADJ || !diag) ? pm.y : -1;
-                        nn[bb][q] = sl >= 0 ? tu[sl] : 0;
-                        xp[bb][q][0] = xp[bb][q][1] = xm[bb][q][0] = xm[bb][q][1] = make_double2(0.0, 0.0);
-                        if (vp >= 0) ld256(p.in + (int64_t)vp * (2 * P) + 2 * lt, xp[bb][q][0], xp[bb][q][1]);
-                        if (vm >= 0) ld256(p.in + (int64_t)vm * (2 * P) + 2 * lt, xm[bb][q][0], xm[bb][q][1]);
-                    }
+            for (int b = 0; b < QB; ++b) {
+                const int q = q0 + b;
+                if (vk[b] >= 0) {
+                    const double2* sq = s_sq + tu[slo[q]];
+                    const double sk = ADJ ? sq->y : sq->x;
+                    auto kap = [&](const double2* tab) {
+                        const double2 v = tab[kp[q]];
+                        return make_double2(v.x * sk, (ADJ ? -v.y : v.y) * sk);
+                    };
+                    cmac(of, kap(kt_of), xo[b][0]);
+                    cmac(gs, kap(kt_gs), xg[b][1]);
+                    const double2 k = kap(kt_j);
+                    if (!dga) cmac(os, k, xo[b][1]);
+                    if (!dgb) cmac(gf, k, xg[b][0]);
                 }
+            }
+            // ---- C neighbours (a diagonal element's terms of its row and column cancel) ----
 #pragma unroll
-                for (int bb = 0; bb < SB; ++bb) {
-                    const int sd = sd0 + bb;
+            for (int b = 0; b < QB; ++b) {
+                const int64_t o = (int64_t)vc[b] * (2 * P);
+                if (vc[b] >= 0) {
+                    ld256_if(no_co, in_o + o, xo[b][0], xo[b][1]);
+                    ld256_if(no_cg, in_g + o, xg[b][0], xg[b][1]);
+                }
+            }
 #pragma unroll
-                    for (int q = 0; q < SLT; ++q) {
-                        const int sl = sd == 0 ? sli[q] : slj[q];
-                        if (sl < 0) continue;
-                        const int ps = s_pos[sl];
-                        const double2 sqp = s_sq[nn[bb][q]];
-                        const double sq_lo = sqp.x, sq_hi = sqp.y;
-                        // L: i chat sqrt(n+1) on the plus neighbour, khat sqrt(n) on the minus one;
-                        // L^H: -i chat sqrt(n) on the minus neighbour, conj(khat) sqrt(n+1) on the plus one
-                        const double c = diag ? 0.0 : (ADJ ? -s_ch[ps] * sq_lo : s_ch[ps] * sq_hi);
-                        const double sk = ADJ ? sq_hi : sq_lo;
-                        const double2 t1 = ADJ ? xm[bb][q][0] : xp[bb][q][0], t2 = ADJ ? xm[bb][q][1] : xp[bb][q][1];
-                        const double2 k1 = ADJ ? xp[bb][q][0] : xm[bb][q][0], k2 = ADJ ? xp[bb][q][1] : xm[bb][q][1];
-                        const double2 m1 = make_double2(k1.x * sk, k1.y * sk);
-                        const double2 m2 = make_double2(k2.x * sk, k2.y * sk);
-                        auto kap = [&](const double2* tab) {
-                            const double2 v = tab[ps];
-                            return ADJ ? make_double2(v.x, -v.y) : v;
-                        };
-                        if (sd == 0) {
-                            // site i: element 1 (i,j) i-side (+i c, kappa_i); element 2 (j,i) j-side (-i c, kappa_j)
-                            L1.x = fma(-c, t1.y, L1.x);
-                            L1.y = fma(c, t1.x, L1.y);
-                            L2.x = fma(c, t2.y, L2.x);
-                            L2.y = fma(-c, t2.x, L2.y);
-                            cmac(L1, kap(kap_i1), m1);
-                            if (!diag) cmac(L2, kap(kap_i2), m2);
-                        } else {
-                            // site j: element 1 j-side (-i c, kappa_j); element 2 i-side (+i c, kappa_i)
-                            L1.x = fma(c, t1.y, L1.x);
-                            L1.y = fma(-c, t1.x, L1.y);
-                            L2.x = fma(-c, t2.y, L2.x);
-                            L2.y = fma(c, t2.x, L2.y);
-                            if (!diag) cmac(L1, kap(kap_j1), m1);
-                            cmac(L2, kap(kap_j2), m2);
-                        }
+            for (int b = 0; b < QB; ++b) {
+                const int q = q0 + b;
+                if (vc[b] >= 0) {
+                    const double2 sq = s_sq[tu[slo[q]]];
+                    const double c = ADJ ? -s_ch[kp[q]] * sq.x : s_ch[kp[q]] * sq.y;
+                    if (!dga) {
+                        of.x = fma(-c, xo[b][0].y, of.x);
+                        of.y = fma(c, xo[b][0].x, of.y);
+                        os.x = fma(c, xo[b][1].y, os.x);
+                        os.y = fma(-c, xo[b][1].x, os.y);
+                    }
+                    if (!dgb) {
+                        gf.x = fma(c, xg[b][0].y, gf.x);
+                        gf.y = fma(-c, xg[b][0].x, gf.y);
+                        gs.x = fma(-c, xg[b][1].y, gs.x);
+                        gs.y = fma(c, xg[b][1].x, gs.y);
                     }
                 }
             }
-
         }
+        if (holds) {
+            hnd[rid] = gf;
+            hnd[TT + rid] = gs;
+        }
+        cp_async_wait_all();
         team_sync<TW>(team);
+        if (more) load_k(slot_n, 0); // in flight through the stores and the next commutator
 
-        if (active) {
-            // ---- commutator: i * (w H - H w) / hbar from the exchange tile ----
-            const double2 c1 = xch[i1 * kXchStride + j1], c2 = xch[i2 * kXchStride + j2];
-            L1.x -= c1.y;
-            L1.y += c1.x;
-            L2.x -= c2.y;
-            L2.y += c2.x;
+        if (owner) {
+            // ---- commutator i * (w H - H w) / hbar and the terms handed over ----
+            const double2 c1 = xch[xc1], c2 = xch[xc2], hf = hnd[lt], hs = hnd[TT + lt];
+            const double2 L1 = make_double2((of.x - c1.y) + hf.x, (of.y + c1.x) + hf.y);
+            double2 L2 = make_double2((os.x - c2.y) + hs.x, (os.y + c2.x) + hs.y);
+            if (ODD && dga && r == N - 1) L2 = L1; // the padding half mirrors its element
 
             // ---- stage write ----
-            const int64_t off = u * (2 * P) + 2 * lt;
-            double2 x1 = s1, x2 = s2;
+            const int64_t off = (int64_t)u * (2 * P) + 2 * pso;
+            double2 x1 = xf, x2 = xs;
             if (p.y) ld256_cg(p.y + off, x1, x2);
             double2 r1 = p.use_x ? x1 : make_double2(0.0, 0.0), r2 = p.use_x ? x2 : make_double2(0.0, 0.0);
             cmac(r1, p.beta, L1);
             cmac(r2, p.beta, L2);
             st256_cs(p.out + off, r1, r2);
             if (p.use_acc) {
-                double2 a1 = s1, a2 = s2;
+                double2 a1 = xf, a2 = xs;
                 if (!p.acc_init) ld256_cg(p.acc + off, a1, a2);
                 cmac(a1, p.acc_beta, L1);
                 cmac(a2, p.acc_beta, L2);
                 st256(p.acc + off, a1, a2);
             }
         }
-        cp_async_wait_all();
-        team_sync<TW>(team);
-        cur ^= 1;
-        ci = ni;
     }
 }
 

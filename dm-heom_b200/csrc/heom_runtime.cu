@@ -549,8 +549,6 @@ int allow_dynamic_smem(const void* fn, size_t smem)
     return 0;
 }
 
-int cta_threads(int n) { return (heomk::kCtaWarps / heomk::team_warps(n)) * heomk::team_warps(n) * 32; }
-int cta_teams(int n) { return heomk::kCtaWarps / heomk::team_warps(n); }
 
 // resolve the launch shape of the stage kernel (outside of any stream capture)
 int resolve_stage(heom_handle* h, const void** fn_out, int* blocks_out = nullptr, bool adj = false, bool gen = false)
@@ -570,7 +568,7 @@ int resolve_stage(heom_handle* h, const void** fn_out, int* blocks_out = nullptr
     } else {
         fn = (const void*)pick_stage(h->N, h->hkind, h->SL == 1 ? 1 : h->SLT, adj); // one slot: exact
         smem = heomk::pair_smem_bytes(h->N, h->W, h->NW, h->TWB, h->LS);
-        threads = cta_threads(h->N);
+        threads = heomk::team_threads(h->N);
     }
     if (!fn) return fail(HEOM_E_UNSUPPORTED, "states = %d not supported", h->N);
     int& per_sm = h->per_sm[adj ? 1 : gen ? 2 : 0][h->hkind];
@@ -580,7 +578,7 @@ int resolve_stage(heom_handle* h, const void** fn_out, int* blocks_out = nullptr
         CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem));
         if (per_sm < 1) return fail(HEOM_E_UNSUPPORTED, "stage kernel cannot be resident");
     }
-    const int teams = h->N <= 8 ? heomk::kRowWarps : cta_teams(h->N);
+    const int teams = h->N <= 8 ? heomk::kRowWarps : heomk::cta_teams(h->N);
     const int64_t groups = h->kp ? h->inst_nodes * (h->kp / 32)
                                  : std::max<int64_t>(1, (h->n_active + teams - 1) / teams);
     const int64_t want = h->grid_override > 0 ? h->grid_override : (int64_t)per_sm * h->sm_count;
@@ -682,7 +680,7 @@ int launch_stage(heom_handle* h, int epi, const double2* in, const double2* y, d
         h->launches++;
         return 0;
     }
-    CUDA_TRY(launch_dependent(fn, blocks, h->N <= 8 ? heomk::kRowWarps * 32 : cta_threads(h->N), h->stage_smem,
+    CUDA_TRY(launch_dependent(fn, blocks, h->N <= 8 ? heomk::kRowWarps * 32 : heomk::team_threads(h->N), h->stage_smem,
                               h->stream, &dp));
     h->launches++;
     return 0;
@@ -999,7 +997,7 @@ int check_same_class(const heom_instance_desc* a, const heom_instance_desc* b)
 }
 
 // sector tables of the pair layout: the searched orders for N <= 8 (row_tables.inc; pair_tables.inc for the
-// lockstep layout), the canonical order of heomk::pair_elements above
+// lockstep layout), the team kernel's order above
 int build_pair_tables(heom_handle* h, bool lockstep = false)
 {
     const int N = h->N, P = h->P;
@@ -1010,7 +1008,16 @@ int build_pair_tables(heom_handle* h, bool lockstep = false)
             e1 = lockstep ? kPairE1[N][p] : kRowE1[N][p];
             e2 = lockstep ? kPairE2[N][p] : kRowE2[N][p];
         } else {
+            // in the order of the team kernel's owners, the owner's row first
             heomk::pair_elements(N, p, &e1, &e2, &i, &j, &d);
+            if (!d && j != 2 * (j / 2) + heomk::row_owned(i, j / 2)) {
+                std::swap(e1, e2);
+                std::swap(i, j);
+            }
+            const int pos = heomk::team_pos(N, i, j / 2);
+            h->pair_tab[2 * pos] = (int16_t)e1;
+            h->pair_tab[2 * pos + 1] = (int16_t)e2;
+            continue;
         }
         h->pair_tab[2 * p] = (int16_t)e1;
         h->pair_tab[2 * p + 1] = (int16_t)e2;

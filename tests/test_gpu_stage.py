@@ -87,3 +87,24 @@ def test_flow_buffers_are_the_neighbour_terms(n, m, depth):
     assert np.max(np.abs(above + below - (ref - rest))) <= 1e-12 * np.max(np.abs(ref))
     last = np.asarray(prob.graph.tuples).reshape(nodes, -1).sum(axis=1) == depth
     assert np.all(above[last] == 0.0) and np.all(below[0] == 0.0)
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("n,m,depth,bps", [(n, m, 2, 1) for n in range(9, 17) for m in (1, 2)] +
+                         [(9, 3, 2, 1), (10, 5, 1, 1), (16, 3, 1, 1), (11, 1, 2, 2), (12, 2, 1, 2)])
+def test_teams(n, m, depth, bps, cplx):
+    """9 to 16 states: even and odd counts (threads that own no sector, the padding half), one to eight slots."""
+    prob = problem(n, m, depth, cplx, bps)
+    y = np.random.default_rng(n * 10 + m).normal(size=prob.state_len)
+    step = ho.rk4_step(prob, 0.5e-15, y)
+    for scheme in ("product", "horner"):
+        with hb.Heom.from_problem(prob, scheme=scheme) as H:
+            H.set_state(y)
+            H.rk4_steps(0.5e-15, 1)
+            got = H.get_state()
+            assert rel(got, step) <= TOL
+    with hb.Heom.batch([hb.Heom.tables_of(prob)] * 2) as H:  # the fragments of an instance per ADO
+        H.set_state(np.concatenate([y, 2.0 * y]))
+        H.rk4_steps(0.5e-15, 1)
+        both = H.get_state()
+    assert rel(both[:y.size], step) <= TOL and rel(both[y.size:], 2.0 * step) <= TOL
