@@ -1226,7 +1226,12 @@ struct GradParams {
     const double* __restrict__ dchat;  // [2][W] d chat
     const double2* __restrict__ dkhat; // [2][3][W] d khat (side i, side j, diagonal)
     const double* __restrict__ sq;     // [LS+1] sqrt(n)
-    double2 weight;                    // beta_k h
+    // one launch takes `factors` pairs (a, w) that follow one another in the backward sweep: pair f at a + f a_step,
+    // w + f w_step (double2 elements), its weight beta_k h with k = factor0 - f (mod 4)
+    int factors, factor0;
+    int64_t a_step, w_step;
+    double2 weight[4];
+    RowTab rt;                         // heom_row_grad
     double2* partial;                  // [gridDim.x][N*N + 2]
     const int64_t* inst_base;          // [instances + 1] first ADO of every instance
     int blocks_per_inst;               // blocks [k*bpi, (k+1)*bpi) sweep instance k only
@@ -1238,10 +1243,10 @@ struct GradParams {
 __host__ __device__ inline int grad_warp_bytes(int n) { return 2 * n * (n + 1) * 16; }
 __host__ inline size_t grad_smem_bytes(int n)
 {
-    return (size_t)kCtaWarps * grad_warp_bytes(n) + (size_t)kCtaWarps * (n * n + 2) * 16;
+    return (size_t)kCtaWarps * grad_warp_bytes(n) + (size_t)(kCtaWarps + 1) * (n * n + 2) * 16;
 }
 
-__global__ void __launch_bounds__(kCtaWarps * 32) heom_adjoint_grad(const GradParams g)
+__global__ void __launch_bounds__(kCtaWarps * 32) heom_adjoint_grad(const __grid_constant__ GradParams g)
 {
     extern __shared__ __align__(128) unsigned char smem[];
     const int N = g.N, P = g.P, W = g.W, SL = g.SL, NN = N * N;
@@ -1255,15 +1260,21 @@ __global__ void __launch_bounds__(kCtaWarps * 32) heom_adjoint_grad(const GradPa
     const int gq = lane >> 2, t4 = lane & 3;
     const int nblk = N <= 8 ? 1 : 4, ks = (N + 3) / 4;
     double zr[4][2], zi[4][2];
-#pragma unroll
-    for (int b = 0; b < 4; ++b) zr[b][0] = zr[b][1] = zi[b][0] = zi[b][1] = 0.0;
-    double2 dl = make_double2(0.0, 0.0), dgm = dl;
     auto el = [&](const double2* T, int r, int c) {
         return (r < N && c < N) ? T[r * (N + 1) + c] : make_double2(0.0, 0.0);
     };
 
     const int inst = blockIdx.x / g.blocks_per_inst, jb = blockIdx.x - inst * g.blocks_per_inst;
     const int64_t stride = (int64_t)g.blocks_per_inst * kCtaWarps, end = g.inst_base[inst + 1];
+    double2* acc = red + kCtaWarps * (NN + 2); // [NN+2]
+    double2* const out = g.partial + (int64_t)blockIdx.x * (NN + 2);
+    for (int q = threadIdx.x; q < NN + 2; q += blockDim.x) acc[q] = out[q];
+    for (int f = 0; f < g.factors; ++f) {
+    const double2* a_in = g.a + f * g.a_step;
+    const double2* w_in = g.w + f * g.w_step;
+#pragma unroll
+    for (int b = 0; b < 4; ++b) zr[b][0] = zr[b][1] = zi[b][0] = zi[b][1] = 0.0;
+    double2 dl = make_double2(0.0, 0.0), dgm = dl;
     for (int64_t u = g.inst_base[inst] + (int64_t)jb * kCtaWarps + warp; u < end; u += stride) {
         const unsigned char* nb = g.rec + u * rec_bytes(g.NW, g.TWB);
         const unsigned char* tu = nb + g.NW * 4;
@@ -1272,8 +1283,8 @@ __global__ void __launch_bounds__(kCtaWarps * 32) heom_adjoint_grad(const GradPa
             const int e1 = g.pe[2 * p], e2 = g.pe[2 * p + 1];
             const int i1 = e1 / N, j1 = e1 - i1 * N, i2 = e2 / N, j2 = e2 - i2 * N;
             double2 a1, a2, w1, w2;
-            ld256(g.a + (u * P + p) * 2, a1, a2);
-            ld256(g.w + (u * P + p) * 2, w1, w2);
+            ld256(a_in + (u * P + p) * 2, a1, a2);
+            ld256(w_in + (u * P + p) * 2, w1, w2);
             At[i1 * (N + 1) + j1] = a1;
             At[i2 * (N + 1) + j2] = a2;
             Wt[i1 * (N + 1) + j1] = w1;
@@ -1301,8 +1312,8 @@ __global__ void __launch_bounds__(kCtaWarps * 32) heom_adjoint_grad(const GradPa
                     const int32_t vp = diag ? -1 : pm.x;
                     const int32_t vm = pm.y;
                     double2 p1 = make_double2(0.0, 0.0), p2 = p1, m1 = p1, m2 = p1;
-                    if (vp >= 0) ld256(g.w + ((int64_t)vp * P + p) * 2, p1, p2);
-                    if (vm >= 0) ld256(g.w + ((int64_t)vm * P + p) * 2, m1, m2);
+                    if (vp >= 0) ld256(w_in + ((int64_t)vp * P + p) * 2, p1, p2);
+                    if (vm >= 0) ld256(w_in + ((int64_t)vm * P + p) * 2, m1, m2);
                     const double shi = g.sq[n + 1], slo = g.sq[n];
                     for (int th = 0; th < 2; ++th) {
                         const double c = g.dchat[th * W + sl] * shi;
@@ -1398,11 +1409,243 @@ __global__ void __launch_bounds__(kCtaWarps * 32) heom_adjoint_grad(const GradPa
             s.x += red[v * (NN + 2) + q].x;
             s.y += red[v * (NN + 2) + q].y;
         }
-        double2& out = g.partial[(int64_t)blockIdx.x * (NN + 2) + q];
-        out.x += g.weight.x * s.x - g.weight.y * s.y;
-        out.y += g.weight.x * s.y + g.weight.y * s.x;
+        const double2 wgt = g.weight[(g.factor0 - f) & 3];
+        acc[q].x += wgt.x * s.x - wgt.y * s.y;
+        acc[q].y += wgt.x * s.y + wgt.y * s.x;
     }
+    __syncthreads();
+    }
+    for (int q = threadIdx.x; q < NN + 2; q += blockDim.x) out[q] = acc[q];
 }
+
+// ---------------------------------------------------------------------------
+// The same for N <= 8 and at most two slots per state, with the lanes of
+// heom_dmma_stage: lane 4r + t reads its two sectors of the neighbours along
+// the baths of state r.  Of the bath terms it keeps theta-independent sums per
+// slot -- <a, row and column terms> scaled by sqrt(n) or sqrt(n+1) -- and the
+// derivatives of the coefficients enter once per launch and factor.  The next
+// ADO's indices are read one ADO ahead: one round trip per ADO is exposed.
+// Latency bounds it.  7 states, one slot, 6435 ADOs: 8.7 us a factor in launches
+// of twelve, against 17 in launches of one with a lane per sector.
+// ---------------------------------------------------------------------------
+template <int N, int SLT>
+__global__ void __launch_bounds__(kCtaWarps * 32, 2) heom_row_grad(const __grid_constant__ GradParams g)
+{
+    static_assert(N <= 8 && SLT <= 2, "row gradient handles N <= 8 and two slots");
+    constexpr int P = pairs_of(N), NN = N * N, LD = N + 1;
+    constexpr bool ODD = (N & 1) != 0;
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int W = g.W;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double2* At = reinterpret_cast<double2*>(smem + warp * grad_warp_bytes(N)); // [N][N+1]
+    double2* Wt = At + N * LD;
+    double2* red = reinterpret_cast<double2*>(smem + kCtaWarps * grad_warp_bytes(N)); // [warps][NN+2]
+    double2* acc = red + kCtaWarps * (NN + 2);                                         // [NN+2]
+
+    // ---- this lane's place (heom_dmma_stage) ----
+    const int r = lane >> 2, t = lane & 3;
+    const int odd = row_owned(r, t);
+    const bool dga = t == (r >> 1) && !(r & 1), dgb = t == (r >> 1) && (r & 1);
+    const int ps0 = opaque(g.rt.pos[lane][0]), ps1 = opaque(g.rt.pos[lane][1]);
+    const int pso = odd ? ps1 : ps0, psg = odd ? ps0 : ps1;
+    const bool owner = pso >= 0, holds = psg >= 0;
+    const int co = 2 * t + odd, cg = 2 * t + 1 - odd;
+    const int i2 = dga ? (r + 1 < N ? r + 1 : r) : co, j2 = dga ? i2 : r; // second element of the owned sector
+    const bool twin = ODD && dga && r == N - 1;                            // padding half
+    const int no_o = owner ? 0 : -1, no_g = holds ? 0 : -1;
+    const int no_co = dga ? -1 : no_o, no_cg = dgb ? -1 : no_g;
+    // tile positions: owned sector's halves, row and column element of the handed-over one
+    const int q1 = owner ? r * LD + co : 0, q2 = owner ? i2 * LD + j2 : 0;
+    const int gr = holds ? r * LD + cg : 0, gc = holds ? (dgb ? gr : cg * LD + r) : 0;
+    int sl[SLT];
+#pragma unroll
+    for (int q = 0; q < SLT; ++q) sl[q] = (r < N && q < g.SL) ? g.slots[r * g.SL + q] : -1;
+    auto el = [&](const double2* T, int i, int j) {
+        return (N == 8 || (i < N && j < N)) ? T[i * LD + j] : make_double2(0.0, 0.0);
+    };
+    auto conj_mac = [](double2& s, const double2 a, const double2 w) { // s += conj(a) w
+        s.x = fma(a.x, w.x, s.x);
+        s.x = fma(a.y, w.y, s.x);
+        s.y = fma(a.x, w.y, s.y);
+        s.y = fma(-a.y, w.x, s.y);
+    };
+
+    const int inst = blockIdx.x / g.blocks_per_inst, jb = blockIdx.x - inst * g.blocks_per_inst;
+    const unsigned stride = (unsigned)g.blocks_per_inst * kCtaWarps, end = (unsigned)g.inst_base[inst + 1];
+    const unsigned begin = (unsigned)g.inst_base[inst] + (unsigned)jb * kCtaWarps + warp;
+    const int recb = rec_bytes(g.NW, g.TWB);
+    double2* const out = g.partial + (int64_t)blockIdx.x * (NN + 2);
+    for (int q = threadIdx.x; q < NN + 2; q += blockDim.x) acc[q] = out[q];
+
+    for (int f = 0; f < g.factors; ++f) {
+        const double2* a_in = g.a + f * g.a_step;
+        const double2* w_in = g.w + f * g.w_step;
+        const double2 z0 = make_double2(0.0, 0.0);
+        double zr0 = 0.0, zr1 = 0.0, zi0 = 0.0, zi1 = 0.0; // Z(r, 2t), Z(r, 2t+1)
+        double2 sp[SLT], si[SLT], sj[SLT], y1 = z0, y2 = z0, sd = z0;
+#pragma unroll
+        for (int q = 0; q < SLT; ++q) sp[q] = si[q] = sj[q] = z0;
+        int2 pm[SLT];
+        int nn[SLT];
+        auto index = [&](unsigned u) {
+            const unsigned char* rec = g.rec + (int64_t)u * recb;
+#pragma unroll
+            for (int q = 0; q < SLT; ++q) {
+                pm[q] = make_int2(-1, -1);
+                nn[q] = 0;
+                if (g.want_bath && sl[q] >= 0 && u < end) {
+                    pm[q] = __ldg(reinterpret_cast<const int2*>(rec) + sl[q]);
+                    nn[q] = rec[g.NW * 4 + sl[q]];
+                }
+            }
+        };
+        index(begin);
+        for (unsigned u = begin; u < end; u += stride) {
+            double2 a1 = z0, a2 = z0, w1 = z0, w2 = z0;
+            double2 xo[2], xg[2]; // minus neighbour
+            const int64_t o = (int64_t)u * (2 * P);
+            if (owner) {
+                ld256_cg(a_in + o + 2 * pso, a1, a2);
+                ld256_cg(w_in + o + 2 * pso, w1, w2);
+            }
+            const double dps = g.dpss[u];
+            int2 cm[SLT];
+            int cn[SLT];
+#pragma unroll
+            for (int q = 0; q < SLT; ++q) {
+                cm[q] = pm[q];
+                cn[q] = nn[q];
+            }
+            auto minus = [&](int q) {
+                const int64_t om = (int64_t)cm[q].y * (2 * P);
+                ld256_if(cm[q].y | no_o, w_in + om + 2 * (owner ? pso : 0), xo[0], xo[1]);
+                ld256_if(cm[q].y | no_g, w_in + om + 2 * (holds ? psg : 0), xg[0], xg[1]);
+            };
+            minus(0);
+            index(u + stride);
+            if (owner) {
+                At[q1] = a1;
+                At[q2] = a2;
+                Wt[q1] = w1;
+                Wt[q2] = w2;
+            }
+            __syncwarp();
+            // Z(k,l) = sum_i w(i,k) conj(a(i,l)) - sum_j conj(a(k,j)) w(l,j):
+            //   Re Z = Wr^T Ar + Wi^T Ai - Ar Wr^T - Ai Wi^T, Im Z = Wi^T Ar - Wr^T Ai - Ar Wi^T + Ai Wr^T
+            if (g.want_h) {
+#pragma unroll
+                for (int s = 0; s < 2; ++s) {
+                    if (4 * s >= N) continue;
+                    const int k0 = 4 * s + t;
+                    const double2 wT = el(Wt, k0, r); // A operand of W^T A: W(4s+t, r)
+                    const double2 aB = el(At, k0, r); // B operand of W^T A: A(4s+t, r)
+                    const double2 aA = el(At, r, k0); // A operand of A W^T: A(r, 4s+t)
+                    const double2 wB = el(Wt, r, k0); // B operand of A W^T: W(r, 4s+t)
+                    dmma(zr0, zr1, wT.x, aB.x);
+                    dmma(zr0, zr1, wT.y, aB.y);
+                    dmma(zr0, zr1, -aA.x, wB.x);
+                    dmma(zr0, zr1, -aA.y, wB.y);
+                    dmma(zi0, zi1, wT.y, aB.x);
+                    dmma(zi0, zi1, -wT.x, aB.y);
+                    dmma(zi0, zi1, -aA.x, wB.y);
+                    dmma(zi0, zi1, aA.y, wB.x);
+                }
+            }
+            if (g.want_bath) {
+                // same term of the owned elements (a padding half counts once)
+                double2 v1 = z0, v2 = z0;
+                conj_mac(v1, a1, w1);
+                if (!twin) conj_mac(v2, a2, w2);
+                y1.x += v1.x;
+                y1.y += v1.y;
+                y2.x += v2.x;
+                y2.y += v2.y;
+                sd.x = fma(dps, v1.x + v2.x, sd.x);
+                sd.y = fma(dps, v1.y + v2.y, sd.y);
+                const double2 ar = At[gr], ac = At[gc]; // handed-over sector: row and column element
+#pragma unroll
+                for (int q = 0; q < SLT; ++q) {
+                    if (q > 0) minus(q);
+                    if (cm[q].y >= 0) {
+                        const double s = g.sq[cn[q]];
+                        double2 vi = z0, vj = z0;
+                        if (owner) {
+                            conj_mac(vi, a1, xo[0]);
+                            conj_mac(vj, dga ? a1 : a2, dga ? xo[0] : xo[1]);
+                        }
+                        if (holds) {
+                            conj_mac(vi, ar, xg[1]);
+                            conj_mac(vj, ac, dgb ? xg[1] : xg[0]);
+                        }
+                        si[q].x = fma(s, vi.x, si[q].x);
+                        si[q].y = fma(s, vi.y, si[q].y);
+                        sj[q].x = fma(s, vj.x, sj[q].x);
+                        sj[q].y = fma(s, vj.y, sj[q].y);
+                    }
+                    if (cm[q].x >= 0) {
+                        const int64_t op = (int64_t)cm[q].x * (2 * P);
+                        ld256_if(no_co, w_in + op + 2 * (owner ? pso : 0), xo[0], xo[1]);
+                        ld256_if(no_cg, w_in + op + 2 * (holds ? psg : 0), xg[0], xg[1]);
+                        const double s = g.sq[cn[q] + 1];
+                        double2 vr = z0, vc = z0; // row elements with +i, column elements with -i
+                        if (no_co >= 0) {
+                            conj_mac(vr, a1, xo[0]);
+                            conj_mac(vc, a2, xo[1]);
+                        }
+                        if (no_cg >= 0) {
+                            conj_mac(vr, ar, xg[1]);
+                            conj_mac(vc, ac, xg[0]);
+                        }
+                        sp[q].x = fma(s, vc.y - vr.y, sp[q].x); // i (vr - vc)
+                        sp[q].y = fma(s, vr.x - vc.x, sp[q].y);
+                    }
+                }
+            }
+            __syncwarp();
+        }
+        // the coefficients' derivatives, then the block's sum in a fixed order, times the factor's weight
+        double2* mine = red + warp * (NN + 2);
+        if (r < N && 2 * t < N) mine[r * N + 2 * t] = make_double2(zr0, zi0);
+        if (r < N && 2 * t + 1 < N) mine[r * N + 2 * t + 1] = make_double2(zr1, zi1);
+        double2 d[2] = {z0, sd}; // lambda, gamma
+#pragma unroll
+        for (int th = 0; th < 2; ++th) {
+            if (g.want_bath && owner) {
+                cmac(d[th], g.dg0[th * NN + r * N + co], y1);
+                cmac(d[th], g.dg0[th * NN + i2 * N + j2], y2);
+            }
+#pragma unroll
+            for (int q = 0; q < SLT; ++q) {
+                if (!g.want_bath || sl[q] < 0) continue;
+                const double2* kh = g.dkhat + th * 3 * W + sl[q];
+                const double c = g.dchat[th * W + sl[q]];
+                d[th].x = fma(c, sp[q].x, d[th].x);
+                d[th].y = fma(c, sp[q].y, d[th].y);
+                cmac(d[th], kh[0], si[q]);
+                cmac(d[th], kh[W], sj[q]);
+            }
+            for (int off = 16; off > 0; off >>= 1) {
+                d[th].x += __shfl_down_sync(0xffffffffu, d[th].x, off);
+                d[th].y += __shfl_down_sync(0xffffffffu, d[th].y, off);
+            }
+            if (lane == 0) mine[NN + th] = d[th];
+        }
+        __syncthreads();
+        const double2 wgt = g.weight[(g.factor0 - f) & 3];
+        for (int q = threadIdx.x; q < NN + 2; q += blockDim.x) {
+            double2 s = z0;
+            for (int v = 0; v < kCtaWarps; ++v) {
+                s.x += red[v * (NN + 2) + q].x;
+                s.y += red[v * (NN + 2) + q].y;
+            }
+            acc[q].x += wgt.x * s.x - wgt.y * s.y;
+            acc[q].y += wgt.x * s.y + wgt.y * s.x;
+        }
+        __syncthreads();
+    }
+    for (int q = threadIdx.x; q < NN + 2; q += blockDim.x) out[q] = acc[q];
+}
+
 
 // y[top of instance k] += w * O_k (O_k row-major n x n complex, obs =
 // [instances][n*n]), pair layout; block k.  w = weights[*base + j] (a device

@@ -2633,6 +2633,8 @@ struct heom_adjoint {
     int grid = 0, bpi = 0;     // blocks of the gradient kernel, per instance
     size_t grad_smem = 0;
     DevBuf<double2> cps, seg, scratch, ga, gb, toplog;
+    DevBuf<double2> ring;      // adjoint states of a group of steps (4 group of them; small hierarchies)
+    int64_t group = 0;         // steps whose gradient contributions are one launch (0: one launch per factor)
     int64_t cap_cps = 0, cap_seg = 0, cap_rows = 0;
     int64_t mem_limit = 0;     // bytes for the sweep's states (0: free device memory)
     int64_t rec_slots = 0;     // recursive-checkpointing slots of the last sweep (0: sqrt layout)
@@ -2644,6 +2646,7 @@ struct heom_adjoint {
     struct Graphs {
         int64_t len = 0;
         cudaGraphExec_t g[3] = {nullptr, nullptr, nullptr};
+        int64_t launches[3] = {0, 0, 0};
     };
     std::vector<Graphs> graphs;
     double graph_dt = 0.0;
@@ -2662,6 +2665,8 @@ struct heom_adjoint {
 };
 
 namespace {
+
+constexpr size_t kRingBytes = size_t(64) << 20;
 
 // L^H tables of every instance and the derivative tables (shared bath tables)
 int adj_tables(heom_adjoint* A, const heomhost::system_params& sp)
@@ -2729,7 +2734,26 @@ int adj_tables(heom_adjoint* A, const heomhost::system_params& sp)
     return 0;
 }
 
-int adj_grad(heom_adjoint* A, const double2* a, const double2* w, double2 weight)
+typedef void (*grad_fn_t)(const heomk::GradParams);
+
+// gradient kernel of the handle's sizes
+grad_fn_t pick_grad(int n, int sl)
+{
+    if (sl <= 2) switch (n) {
+#define HEOM_CASE(K) \
+    case K: return sl == 1 ? heomk::heom_row_grad<K, 1> : heomk::heom_row_grad<K, 2>;
+        HEOM_CASE(1) HEOM_CASE(2) HEOM_CASE(3) HEOM_CASE(4) HEOM_CASE(5) HEOM_CASE(6)
+        HEOM_CASE(7) HEOM_CASE(8)
+#undef HEOM_CASE
+    default: break;
+    }
+    return heomk::heom_adjoint_grad;
+}
+
+// gradient contributions of `factors` pairs that follow one another in the backward sweep, the first (factor k0 of
+// its step) with adjoint a and stage input w, the later ones a_step and w_step elements on
+int adj_grad(heom_adjoint* A, const double2* a, const double2* w, double dt, int k0, int factors = 1,
+             int64_t a_step = 0, int64_t w_step = 0)
 {
     heom_handle* h = A->h;
     heomk::GradParams g{};
@@ -2743,7 +2767,12 @@ int adj_grad(heom_adjoint* A, const double2* a, const double2* w, double2 weight
     g.dchat = A->dchat.p;
     g.dkhat = A->dkhat.p;
     g.sq = h->d_sq.p;
-    g.weight = weight;
+    for (int k = 0; k < 4; ++k) g.weight[k] = make_double2(dt * kProdBeta[k][0], dt * kProdBeta[k][1]);
+    g.factors = factors;
+    g.factor0 = k0;
+    g.a_step = a_step;
+    g.w_step = w_step;
+    g.rt = h->row_tab;
     g.partial = A->partial.p;
     g.inst_base = A->inst_base.p;
     g.blocks_per_inst = A->bpi;
@@ -2755,7 +2784,7 @@ int adj_grad(heom_adjoint* A, const double2* a, const double2* w, double2 weight
     g.SL = h->SL;
     g.want_h = A->want_h;
     g.want_bath = A->want_bath;
-    heomk::heom_adjoint_grad<<<A->grid, heomk::kCtaWarps * 32, A->grad_smem, h->stream>>>(g);
+    pick_grad(h->N, h->SL)<<<A->grid, heomk::kCtaWarps * 32, A->grad_smem, h->stream>>>(g);
     h->launches++;
     CUDA_TRY(cudaGetLastError());
     return 0;
@@ -2804,19 +2833,42 @@ int adj_seg_recompute(heom_adjoint* A, double dt, int64_t len)
 }
 
 // backward through a segment: four factors per step (gradient contributions,
-// then F_k^H), then the step's loss weight; the adjoint ends in ga (4 swaps a step)
+// then F_k^H), then the step's loss weight; the adjoint ends where it began.
+// With a ring of 4 G adjoint states the gradient contributions of G steps are
+// one launch: the factors of a group leave their adjoints in the ring, and its
+// last one, after that launch, writes the ring's first state again.
 int adj_seg_backward(heom_adjoint* A, double dt, int64_t len)
 {
     heom_handle* h = A->h;
     const size_t st = h->state_elems();
+    auto factor = [&](const double2* in, double2* out, int k) {
+        return launch_stage(h, EPI_AXPY_SELF, in, nullptr, out, nullptr,
+                            make_double2(dt * kProdBeta[k][0], -dt * kProdBeta[k][1]), 0, &A->tabs);
+    };
+    if (A->group > 0) {
+        double2* ring = A->ring.p;
+        for (int64_t j = len; j > 0;) { // steps j - 1, j - 2, ... of the segment
+            const int64_t steps = std::min<int64_t>(j, A->group), m = 4 * steps;
+            for (int64_t f = 0; f < m; ++f) {
+                const bool last = f + 1 == m;
+                if (last)
+                    if (int rc = adj_grad(A, ring, A->seg.p + (4 * j - 1) * st, dt, 3, (int)m, (int64_t)st, -(int64_t)st))
+                        return rc;
+                double2* out = last ? ring : ring + (f + 1) * st;
+                if (int rc = factor(ring + f * st, out, 3 - (int)(f & 3))) return rc;
+                if ((f & 3) == 3)
+                    if (int rc = adj_add_top(A, out, j - 1 - f / 4)) return rc;
+            }
+            j -= steps;
+        }
+        return 0;
+    }
     double2* gcur = A->ga.p;
     double2* gnxt = A->gb.p;
     for (int64_t j = len - 1; j >= 0; --j) {
         for (int k = 3; k >= 0; --k) {
-            const double2 beta = make_double2(dt * kProdBeta[k][0], dt * kProdBeta[k][1]);
-            if (int rc = adj_grad(A, gcur, A->seg.p + (4 * j + k) * st, beta)) return rc;
-            const double2 cbeta = make_double2(beta.x, -beta.y);
-            if (int rc = launch_stage(h, EPI_AXPY_SELF, gcur, nullptr, gnxt, nullptr, cbeta, 0, &A->tabs)) return rc;
+            if (int rc = adj_grad(A, gcur, A->seg.p + (4 * j + k) * st, dt, k)) return rc;
+            if (int rc = factor(gcur, gnxt, k)) return rc;
             std::swap(gcur, gnxt);
         }
         if (int rc = adj_add_top(A, gcur, j)) return rc;
@@ -2852,6 +2904,7 @@ int adj_run(heom_adjoint* A, int which, double dt, int64_t len)
         CUDA_TRY(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
         const int rc = direct();
         cudaError_t ce = cudaStreamEndCapture(h->stream, &graph);
+        e->launches[which] = h->launches - saved;
         h->launches = saved;
         if (rc) {
             if (graph) cudaGraphDestroy(graph);
@@ -2863,7 +2916,7 @@ int adj_run(heom_adjoint* A, int which, double dt, int64_t len)
         if (ce != cudaSuccess) return fail(HEOM_E_CUDA, "adjoint graph instantiate failed: %s", cudaGetErrorString(ce));
     }
     CUDA_TRY(cudaGraphLaunch(e->g[which], h->stream));
-    h->launches += which == 0 ? len * (launches_per_step(h) + 1) : which == 1 ? 4 * len : 9 * len;
+    h->launches += e->launches[which];
     return 0;
 }
 
@@ -3021,7 +3074,7 @@ int heom_adjoint_create_batch(const heom_system_desc* systems, int32_t count, co
     if (int rc = A->inst_base.alloc(count + 1)) return rc;
     CUDA_TRY(cudaMemcpy(A->inst_base.p, h->inst_base.data(), (count + 1) * 8, cudaMemcpyHostToDevice));
     A->grad_smem = heomk::grad_smem_bytes(h->N);
-    if (int rc = allow_dynamic_smem((const void*)heomk::heom_adjoint_grad, A->grad_smem)) return rc;
+    if (int rc = allow_dynamic_smem((const void*)pick_grad(h->N, h->SL), A->grad_smem)) return rc;
     *out = A.release();
     return 0;
 }
@@ -3075,6 +3128,27 @@ int heom_adjoint_gradient(heom_adjoint* A, const double* rho0, const double* obs
         }
     }
     A->rec_slots = slots;
+    // Small hierarchies: the gradient launches of a few steps are one, over a ring of adjoint states of at most
+    // kRingBytes. A launch over 6435 ADOs leaves a warp three of them and is prologue, tail and latency (7 sites, depth
+    // 8: 17 us a factor alone); from 16 MB a state a launch fills the device by itself. The ring takes no room from the
+    // checkpoints.
+    int64_t group = 0;
+    if (slots == 0 && A->mem_limit == 0) {
+        const size_t sb = st * 16;
+        group = std::min<int64_t>(S, (int64_t)(kRingBytes / (4 * sb)));
+        size_t free_b = 0, total_b = 0;
+        CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
+        if (A->ring.n < 4 * (size_t)group * st && free_b < (size_t)(ncp + 4 * S + 3) * sb + 2 * kRingBytes) group = 0;
+    }
+    if (group != A->group) {
+        A->drop_graphs();
+        A->group = group;
+        if (4 * (size_t)group * st > A->ring.n || group == 0) {
+            A->ring.reset();
+            if (group > 0)
+                if (int rc = A->ring.alloc(4 * (size_t)group * st)) return rc;
+        }
+    }
     // the gradients to accumulate (NULL outputs are skipped); the captured graphs hold them
     const int want_h = grad_h ? 1 : 0, want_bath = (grad_lambda || grad_gamma) ? 1 : 0;
     if (want_h != A->want_h || want_bath != A->want_bath) {
@@ -3178,7 +3252,7 @@ int heom_adjoint_gradient(heom_adjoint* A, const double* rho0, const double* obs
     }
 
     // ---- backward (sqrt layout; the recursive sweep has run above) ----
-    double2* gcur = A->ga.p;
+    double2* gcur = A->group > 0 ? A->ring.p : A->ga.p; // adj_seg_backward's state between segments
     if (slots == 0) {
         CUDA_TRY(cudaMemsetAsync(A->partial.p, 0, (size_t)A->grid * (NN + 2) * 16, h->stream));
         CUDA_TRY(cudaMemsetAsync(gcur, 0, st * 16, h->stream));
