@@ -6,16 +6,15 @@ An ADO (N x N complex) is stored as P = N(N-1)/2 + ceil(N/2) sectors of
 elements.  The lockstep kernel computes the commutator of every instance with
 FP64 m8n8k4 MMAs on the tile zero-padded to 8 x 8: lane l = 4r + t reads, for
 k-slice s, the sector of the pair {r, k}, k = 2t + s, whose two halves are
-exactly its A-fragment element (r, k) and its B-fragment element (k, r).  The MMA result (r, 2t), (r, 2t+1) goes through a
-swizzled row-major tile in shared memory (chunk = 8 r + (c ^ swz(r))) to the
-lane that owns the sector.
+exactly its A-fragment element (r, k) and its B-fragment element (k, r).
 
 This script searches (simulated annealing) the sector numbering and the
 orientation of each pair so that
   * the fragment reads of every quarter warp hit 8 different 16-byte bank
     groups (no shared-memory bank conflicts); for N = 8 also with the slices
     k = 4s + t (a rule of the layout check, weighed above the others),
-  * the exchange reads (owner lane p reading C(e1), C(e2)) are conflict free,
+  * lane p reading the elements of sector p from a row-major tile (chunk =
+    8 r + (c ^ swz(r))) is conflict free (a rule of the layout check too),
   * secondarily (a tie-break), the sectors of each bath's cross (row b and
     column b) fall into few 128-byte lines.
 The result is deterministic for the fixed seeds below.

@@ -175,11 +175,6 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem)
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
 }
-__device__ __forceinline__ void cp_async4(void* smem, const void* gmem)
-{
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem) : "memory");
-}
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 template <int TW>
@@ -199,8 +194,6 @@ __device__ __forceinline__ void cmac(double2& acc, const double2 a, const double
     acc.y = fma(a.x, b.y, acc.y);
     acc.y = fma(a.y, b.x, acc.y);
 }
-
-__device__ __forceinline__ double2 ldg2(const double2* p) { return __ldg(p); }
 
 // ---------------------------------------------------------------------------
 // N <= 8: one warp per ADO, one lane per (state, column pair).
@@ -365,8 +358,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity)
     }
     return false;
 }
-
-__device__ __forceinline__ int swz(int r) { return ((r & 1) << 2) | (r & 1) | (((r >> 1) & 1) << 1); }
 
 // bytes of one pipeline slot and of a warp's shared area for the DMMA kernel:
 // the tile, the ADO's record and 16 bytes of zeros (operands outside N x N)
@@ -765,15 +756,24 @@ __global__ void __launch_bounds__(kRowWarps * 32, row_blocks(HK, SLT, MI)) heom_
 //      [p][32] whose columns are swizzled (k ^ (p & 3)), which keeps the
 //      conflict-free operand reads of the pair order; warp w computes the
 //      commutator of instances w, w+8, w+16, w+24 on the tensor pipe (the
-//      operand mapping and exchange of heom_dmma_stage) and writes the two
-//      commutator values of every sector into a second shared tile;
-//   B  warp w takes sectors w, w+8, ...; lane k is instance k of the block.
+//      operand mapping of heom_dmma_stage); the result of a lane is that of
+//      its own row elements and goes to a second shared tile, to the place
+//      where the lane read them in the first;
+//   B  warp w takes every eighth sector of a list whose first, ninth, ...
+//      entries are the diagonal ones (half the terms: 7 states leave one warp
+//      four of 25 sectors); lane k is instance k of the block.
 //      Neighbour indices, tuple entries and bath coefficients are the same
 //      for every lane (warp-uniform), and each neighbour read is one
 //      contiguous 1-KB row (32 instances x 32 B) of the neighbour ADO, where
 //      heom_dmma_stage gathers 32-B sectors of eight different neighbours.
 // The derivative is the same element by element as heom_dmma_stage's (the
 // same bath-term order; the commutator from the same MMA sequence).
+// Instruction issue and the L1 data pipe bound it.  us per stage, one B200: 256
+// instances of 7 states, depth 6: 245.3 -> 244.3 with the list and absent
+// neighbours skipped (the terms of both sides now add up as heom_dmma_stage's
+// do), -> 225.3 without an exchange of the commutator through shared memory;
+// 40 at depth 4: 18.8 -> 16.3 -> 14.7; 64 of 6 states, two slots, depth 4: 69.5
+// -> 68.7 -> 62.9.
 // ---------------------------------------------------------------------------
 
 // ---------------------------------------------------------------------------
@@ -803,7 +803,7 @@ __global__ void __launch_bounds__(kRowWarps * 32, row_blocks(HK, SLT, MI)) heom_
 // 373 of them shared memory) and the FP64 tensor pipe a quarter.  Measured
 // against a thread per sector with two barriers per ADO (us per stage, one
 // B200): 12 states, two slots, 20,475 ADOs 74.5 -> 55.5 (24 warps of 80
-// registers: 66), one slot, 18,564 ADOs 51.9 -> 43.1; 10 states, two slots,
+// registers: 66) -> 53.4 with y read before the barrier, one slot, 18,564 ADOs 51.9 -> 43.1; 10 states, two slots,
 // 10,626 ADOs 29.4 -> 24.4; 9 states, one slot, 5005 ADOs 13.9 -> 11.8; 11
 // states (three warps instead of two), one slot, 12,376 ADOs 29.3 -> 28.6.
 // ---------------------------------------------------------------------------
@@ -893,7 +893,6 @@ __global__ void __launch_bounds__(team_threads(N), team_blocks(N, HK, SLT))
     double2* hand = reinterpret_cast<double2*>(team_base + L.hand_off);
     for (int q = 0; q < 4; ++q) hand[q * TT + lt] = make_double2(0.0, 0.0);
     __syncthreads();
-    grid_wait(); // the state and the H tables of a field are written by the kernels before this one
 
     const unsigned nodes = (unsigned)p.nodes; // at most 2^31 - 1
     constexpr int TEAMS = cta_teams(N);
@@ -916,24 +915,34 @@ __global__ void __launch_bounds__(team_threads(N), team_blocks(N, HK, SLT))
     // xo, xg the K neighbours' sectors
     int vk[QB], vc[QB];
     double2 xo[QB][2], xg[QB][2];
-    auto load_k = [&](const unsigned char* slot, int q0) {
-        const int2* nb = reinterpret_cast<const int2*>(slot + L.nbr_off);
+    auto index = [&](const unsigned char* rec, int q0) {
+        const int2* nb = reinterpret_cast<const int2*>(rec);
 #pragma unroll
         for (int b = 0; b < QB; ++b) {
             const int2 pm = kp[q0 + b] >= 0 ? nb[slo[q0 + b]] : make_int2(-1, -1);
             vk[b] = ADJ ? pm.x : pm.y;
             vc[b] = ADJ ? pm.y : pm.x;
+        }
+    };
+    auto load_k = [&]() {
+#pragma unroll
+        for (int b = 0; b < QB; ++b) {
             const int64_t o = (int64_t)vk[b] * (2 * P);
             ld256_if(ODD ? vk[b] | no_o : vk[b], in_o + o, xo[b][0], xo[b][1]);
             ld256_if(ODD ? vk[b] | no_g : vk[b], in_g + o, xg[b][0], xg[b][1]);
         }
     };
 
+    // the first ADO's indices come from the record array, so that its neighbours are asked for together with its tile
+    if (u < nodes) index(p.rec + (int64_t)u * recb, 0);
+    grid_wait(); // the state and the H tables of a field are written by the kernels before this one
     unsigned it = 0;
-    if (u < nodes) prefetch(u, team_base);
+    if (u < nodes) {
+        prefetch(u, team_base);
+        load_k();
+    }
     cp_async_wait_all();
     team_sync<TW>(team);
-    if (u < nodes) load_k(team_base, 0);
     for (; u < nodes; u += stride, ++it) {
         const unsigned char* slot = team_base + (it & 1) * L.slot;
         unsigned char* slot_n = team_base + ((it & 1) ^ 1) * L.slot;
@@ -997,9 +1006,16 @@ __global__ void __launch_bounds__(team_threads(N), team_blocks(N, HK, SLT))
             cmac(of, make_double2(pss.x + g1.x, pss.y + g1.y), xf);
             cmac(os, make_double2(pss.x + g2.x, pss.y + g2.y), xs);
         }
+        // what the stage adds to: y takes the place of the own values, in flight through the bath terms (a launch with
+        // y never starts acc from the own values)
+        double2 x1 = xf, x2 = xs;
+        if (p.y && owner) ld256_cg(p.y + (int64_t)u * (2 * P) + 2 * pso, x1, x2);
 #pragma unroll
         for (int q0 = 0; q0 < SLT; q0 += QB) {
-            if (q0 > 0) load_k(slot, q0);
+            if (q0 > 0) {
+                index(slot + L.nbr_off, q0);
+                load_k();
+            }
             // ---- bath terms: K neighbours ----
 #pragma unroll
             for (int b = 0; b < QB; ++b) {
@@ -1054,7 +1070,10 @@ __global__ void __launch_bounds__(team_threads(N), team_blocks(N, HK, SLT))
         }
         cp_async_wait_all();
         team_sync<TW>(team);
-        if (more) load_k(slot_n, 0); // in flight through the stores and the next commutator
+        if (more) { // in flight through the stores and the next commutator
+            index(slot_n + L.nbr_off, 0);
+            load_k();
+        }
 
         if (owner) {
             // ---- commutator i * (w H - H w) / hbar and the terms handed over ----
@@ -1065,14 +1084,12 @@ __global__ void __launch_bounds__(team_threads(N), team_blocks(N, HK, SLT))
 
             // ---- stage write ----
             const int64_t off = (int64_t)u * (2 * P) + 2 * pso;
-            double2 x1 = xf, x2 = xs;
-            if (p.y) ld256_cg(p.y + off, x1, x2);
             double2 r1 = p.use_x ? x1 : make_double2(0.0, 0.0), r2 = p.use_x ? x2 : make_double2(0.0, 0.0);
             cmac(r1, p.beta, L1);
             cmac(r2, p.beta, L2);
             st256_cs(p.out + off, r1, r2);
             if (p.use_acc) {
-                double2 a1 = xf, a2 = xs;
+                double2 a1 = x1, a2 = x2;
                 if (!p.acc_init) ld256_cg(p.acc + off, a1, a2);
                 cmac(a1, p.acc_beta, L1);
                 cmac(a2, p.acc_beta, L2);

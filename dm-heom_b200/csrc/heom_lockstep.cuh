@@ -38,12 +38,15 @@ struct __align__(16) LockSlot {
 struct __align__(16) LockSector {
     int sa, sb, diag, ps;  // sites of side 0 and side 1 (element i1, then j1 or, diagonal, i2); the sector
     double2 g1, g2;        // gamma0 of its two elements
+    int twin, pad[3];      // 1: the second half is the padding half, the first's copy
 };
 __host__ __device__ inline int lock_row_bytes(int NW, int TWB) { return rec_bytes(NW, TWB); }
+// rows of the commutator tile: the sectors, and for N < 8 one for elements outside the N x N block
+__host__ __device__ constexpr int lock_comm_rows(int P) { return P < 32 ? P + 1 : 32; }
 __host__ inline size_t lockstep_smem_bytes(int P, int W, int NW, int TWB, int LS)
 {
-    return (size_t)dmma_lut_bytes(W, LS) + 2 * (size_t)P * 32 * 32 /* two tiles */ + 32 * 32 * 32 /* commutators */ +
-           (size_t)kLockWarps * 64 * 16 + 32 * sizeof(LockSector) + 32 * sizeof(LockSlot) +
+    return (size_t)dmma_lut_bytes(W, LS) + 2 * (size_t)P * 32 * 32 /* two tiles */ +
+           (size_t)lock_comm_rows(P) * 32 * 32 /* commutators */ + 32 * sizeof(LockSector) + 32 * sizeof(LockSlot) +
            2 * (size_t)lock_row_bytes(NW, TWB);
 }
 
@@ -95,9 +98,8 @@ __global__ void __launch_bounds__(kLockWarps * 32, 2) heom_lockstep_stage(const 
         s_sq[q] = make_double2(lp.ct.sq[q], q < LS ? lp.ct.sq[q + 1] : 0.0);
     unsigned char* base = smem + dmma_lut_bytes(W, LS);
     double2* tiles = reinterpret_cast<double2*>(base);      // [2][P][32] sectors (2 double2 each)
-    double2* ctile = tiles + 2 * 2 * P * 32;                 // [32][32] commutator values (rows >= P unused)
-    double2* xch = ctile + 2 * 32 * 32 + (threadIdx.x >> 5) * 64;
-    LockSector* sectors = reinterpret_cast<LockSector*>(ctile + 2 * 32 * 32 + kLockWarps * 64);
+    double2* ctile = tiles + 2 * 2 * P * 32;                 // [P][32] commutator values, one row more for N < 8
+    LockSector* sectors = reinterpret_cast<LockSector*>(ctile + 2 * lock_comm_rows(P) * 32);
     LockSlot* slots = reinterpret_cast<LockSlot*>(sectors + 32);
     unsigned char* rows0 = reinterpret_cast<unsigned char*>(slots + 32);
     const int rowb = lock_row_bytes(p.NW, p.TWB);
@@ -119,6 +121,8 @@ __global__ void __launch_bounds__(kLockWarps * 32, 2) heom_lockstep_stage(const 
         sc.ps = ps;
         sc.g1 = p.gamma0[e1];
         sc.g2 = p.gamma0[e2];
+        sc.twin = e1 == e2 ? 1 : 0;
+        sc.pad[0] = sc.pad[1] = sc.pad[2] = 0;
         sectors[threadIdx.x] = sc;
     }
 
@@ -132,14 +136,9 @@ __global__ void __launch_bounds__(kLockWarps * 32, 2) heom_lockstep_stage(const 
             hbk[j][s] = (HK != H_GENERIC && k < lp.K) ? __ldg(p.hfrag + (size_t)k * 256 + 32 * s + lane) : 0.0;
     }
 
-    const bool owner = lane < P;
-    const int ae1 = opaque(owner ? lp.lt.e1[lane] : 0), ae2 = opaque(owner ? lp.lt.e2[lane] : 0);
-    const int ai1 = ae1 / N, aj1 = ae1 - ai1 * N, ai2 = ae2 / N, aj2 = ae2 - ai2 * N;
     const int fs0 = opaque(lp.lt.fs[lane][0]), fs1 = opaque(lp.lt.fs[lane][1]);
     const int ha0 = opaque(lp.lt.ha[lane][0]), ha1 = opaque(lp.lt.ha[lane][1]);
     const int r = lane >> 2, t = lane & 3;
-    const int xr1 = 8 * ai1 + (aj1 ^ swz(ai1)), xr2 = 8 * ai2 + (aj2 ^ swz(ai2));
-    const int xw0 = 8 * r + ((2 * t) ^ swz(r)), xw1 = 8 * r + ((2 * t + 1) ^ swz(r));
     // Phase A offsets (double2, from a tile buffer) of this lane's operands for the warp's first
     // instance; its instance warp + 8 j adds 16 j, since the column swizzle k ^ (p & 3) changes
     // bits 0-1 of k only. An operand outside the N x N block reads an arbitrary finite tile value
@@ -156,10 +155,9 @@ __global__ void __launch_bounds__(kLockWarps * 32, 2) heom_lockstep_stage(const 
         oa[s] = fs >= 0 ? row + (ha ^ hw) : 0;
         ob[s] = fs >= 0 ? (r == 2 * t + s ? row + (ha ^ hw) : row + (ha ^ 1 ^ hw)) : 0; // diagonal: its own transpose
     }
-    const int oc = (lane * 32 + (warp ^ (lane & 3))) * 2; // this lane's commutator row (lanes >= P: unused rows)
-    // its two commutator stores: first position (lane >> 2) & 1, whichever half lives there
-    const int cpa = (lane >> 2) & 1;
-    const int xra = (cpa ^ hw) == 0 ? xr1 : xr2, xrb = (cpa ^ hw) == 0 ? xr2 : xr1;
+    // the MMA result is the lane's own row elements (r, 2t), (r, 2t+1): the commutator of element (r, 2t+s) goes
+    // where the A operand of slice s was read (elements outside the N x N block: a row that is not read)
+    const int oc0 = fs0 >= 0 ? oa[0] : P * 64, oc1 = fs1 >= 0 ? oa[1] : P * 64;
     const int hk = (lane >> 2) & 1; // phase B: position of half 0 of this lane's instance
     // the slot of site (lane / SLT) that lane of the table warp resolves
     const int tsite = lane / SLT, tq = lane - tsite * SLT;
@@ -273,12 +271,8 @@ __global__ void __launch_bounds__(kLockWarps * 32, 2) heom_lockstep_stage(const 
 #pragma unroll
                 for (int jj = 0; jj < 2; ++jj) {
                     const int j = j0 + jj;
-                    xch[xw0] = make_double2(cr[jj][0], ci[jj][0]);
-                    xch[xw1] = make_double2(cr[jj][1], ci[jj][1]);
-                    __syncwarp();
-                    ctile[oc + 16 * j + cpa] = xch[xra];
-                    ctile[oc + 16 * j + (cpa ^ 1)] = xch[xrb];
-                    __syncwarp();
+                    ctile[oc0 + 16 * j] = make_double2(cr[jj][0], ci[jj][0]);
+                    ctile[oc1 + 16 * j] = make_double2(cr[jj][1], ci[jj][1]);
                 }
             }
         }
@@ -319,7 +313,7 @@ __global__ void __launch_bounds__(kLockWarps * 32, 2) heom_lockstep_stage(const 
                         const int col = (ps * 32 + (lane ^ (ps & 3))) * 2;
                         s1 = tile[col + hk];
                         s2 = tile[col + (hk ^ 1)];
-                        const double2 c1 = ctile[col + hk], c2 = ctile[col + (hk ^ 1)];
+                        const double2 c1 = ctile[col + hk], c2 = ctile[col + (hk ^ 1 ^ sc.twin)];
                         A[0][0] = make_double2(-c1.y, c1.x); // i * (w H - H w) / hbar
                         A[1][1] = make_double2(-c2.y, c2.x);
                         cmac(A[0][0], make_double2(pss.x + sc.g1.x, pss.y + sc.g1.y), s1);
