@@ -90,6 +90,7 @@ struct PairParams {
     int acc_init;
     int use_acc;
     int no_same;                     // leave out pf_same_sum (flow tracking)
+    int same_real;                   // pf_same_sum and gamma0 are real
     // one record of rec_bytes(NW, TWB) per ADO: (plus, minus) of every slot as int32, padded to NW (multiple of 4);
     // the tuple bytes, padded to TWB (multiple of 16); pf_same_sum (double2)
     const unsigned char* __restrict__ rec;
@@ -233,7 +234,9 @@ __device__ __forceinline__ void cmac(double2& acc, const double2 a, const double
 // under register pressure it cost 180 instructions per ADO and half the speed.
 // Two slots: the K neighbours are read one ADO ahead and the coefficients come
 // from shared memory (in registers they spill: 1137 us); one slot: the other
-// way round (15.4 against 16.0 us; 16.9 with both ahead).
+// way round.  Two slots: reading the real parts of the same term's factors alone
+// and the own sector's halves in a staggered order took 13 wavefronts more:
+// 74,613 ADOs 50.1, 735,471 ADOs 540.
 // ---------------------------------------------------------------------------
 
 // which of its two sectors lane (r, t) owns: 0 = {r, 2t}, 1 = {r, 2t+1}
@@ -271,7 +274,7 @@ struct DmmaParams {
     PairParams p;
     RowTab rt; // N <= 8
     CoefTabs ct;
-    int* err;
+    int* err; // mapped host memory
 };
 
 __device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b)
@@ -424,6 +427,7 @@ __global__ void __launch_bounds__(kRowWarps * 32, row_blocks(HK, SLT, MI)) heom_
     constexpr int P = pairs_of(N);
     constexpr bool AHEAD = SLT > 1;            // read the K neighbours one ADO ahead
     constexpr bool XLATE = SLT > 1;            // read the sector's own values again at the end
+    constexpr bool SPLIT = SLT > 1;            // same term: real parts first (one slot: the split spills)
     constexpr bool KREG = SLT == 1;            // coefficients in registers (two slots: they would spill)
     constexpr int QB = SLT < 2 ? SLT : 2;      // slots whose neighbours are read in one batch
     constexpr bool ODD = (N & 1) != 0;         // some lanes hold one sector only
@@ -475,11 +479,14 @@ __global__ void __launch_bounds__(kRowWarps * 32, row_blocks(HK, SLT, MI)) heom_
     const int no_co = dga ? -1 : no_o, no_cg = dgb ? -1 : no_g;
     const double2* in_o = p.in + 2 * (owner ? pso : 0);
     const double2* in_g = p.in + 2 * (holds ? psg : 0);
+    const int xh = (pso & 4) ? 16 : 0; // which half of its own sector a lane reads first (conflict-free quarter warps)
 
     // gamma0 of the lane's row elements ([2][32], the same for every warp)
+    // SPLIT: the real parts of both, then the imaginary parts, which are read only where a bath has some
     if (warp < 2) {
-        const bool in = warp ? ps1 >= 0 : ps0 >= 0;
-        s_g0[threadIdx.x] = in ? p.gamma0[r * N + 2 * t + warp] : make_double2(0.0, 0.0);
+        const double2 z = make_double2(0.0, 0.0);
+        const double2 e0 = ps0 >= 0 ? p.gamma0[r * N + 2 * t] : z, e1 = ps1 >= 0 ? p.gamma0[r * N + 2 * t + 1] : z;
+        s_g0[threadIdx.x] = SPLIT ? (warp ? make_double2(e0.y, e1.y) : make_double2(e0.x, e1.x)) : (warp ? e1 : e0);
     }
     int slo[SLT];                                       // record offsets of the slots of state r: their tuple byte
     int kp[SLT];                                        // table positions of the slots (-1: none)
@@ -632,9 +639,26 @@ __global__ void __launch_bounds__(kRowWarps * 32, row_blocks(HK, SLT, MI)) heom_
             }
             // row elements: i * (w H - H w) / hbar and the same term
             double2 t0 = make_double2(-ci0, cr0), t1 = make_double2(-ci1, cr1);
-            const double2 g0 = s_g0[lane], g1 = s_g0[32 + lane];
-            cmac(t0, make_double2(pss.x + g0.x, pss.y + g0.y), r0);
-            cmac(t1, make_double2(pss.x + g1.x, pss.y + g1.y), r1);
+            if (SPLIT) {
+                const double2 gr = s_g0[lane];
+                const double s0 = pss.x + gr.x, s1 = pss.x + gr.y;
+                t0.x = fma(s0, r0.x, t0.x);
+                t0.y = fma(s0, r0.y, t0.y);
+                t1.x = fma(s1, r1.x, t1.x);
+                t1.y = fma(s1, r1.y, t1.y);
+                if (!p.same_real) {
+                    const double2 gi = s_g0[32 + lane];
+                    const double u0 = pss.y + gi.x, u1 = pss.y + gi.y;
+                    t0.x = fma(-u0, r0.y, t0.x);
+                    t0.y = fma(u0, r0.x, t0.y);
+                    t1.x = fma(-u1, r1.y, t1.x);
+                    t1.y = fma(u1, r1.x, t1.y);
+                }
+            } else {
+                const double2 g0 = s_g0[lane], g1 = s_g0[32 + lane];
+                cmac(t0, make_double2(pss.x + g0.x, pss.y + g0.y), r0);
+                cmac(t1, make_double2(pss.x + g1.x, pss.y + g1.y), r1);
+            }
             of = sel2(odd, t1, t0);
             gs = sel2(odd, t0, t1);
             os = gf = make_double2(0.0, 0.0);
@@ -704,8 +728,10 @@ __global__ void __launch_bounds__(kRowWarps * 32, row_blocks(HK, SLT, MI)) heom_
         if (owner) {
             const int64_t off = (int64_t)u * (2 * P) + 2 * pso;
             if (XLATE) {
-                xf = *reinterpret_cast<const double2*>(slot + (odd ? ro1 : ro0));
-                xs = *reinterpret_cast<const double2*>(slot + (odd ? co1 : co0));
+                const double2 xa = *reinterpret_cast<const double2*>(slot + pso * 32 + xh);
+                const double2 xb = *reinterpret_cast<const double2*>(slot + pso * 32 + (xh ^ 16));
+                xf = sel2(xh == 0, xa, xb);
+                xs = sel2(xh == 0, xb, xa);
             }
             double2 o1 = xf, o2 = xs;
             if (GEN) {
@@ -740,7 +766,7 @@ __global__ void __launch_bounds__(kRowWarps * 32, row_blocks(HK, SLT, MI)) heom_
     }
     // a warp whose wait expired flags the launch as failed and leaves; every copy it issued was either waited
     // for or is the one whose wait has just run to its limit
-    if (failed && lane == 0) atomicExch(dp.err, 1);
+    if (failed && lane == 0) *static_cast<volatile int*>(dp.err) = 1;
 }
 
 // ---------------------------------------------------------------------------
@@ -1856,14 +1882,14 @@ __global__ void heom_hierarchy_norm(double* __restrict__ norms, const double2* _
     }
 }
 
-// Sets *flag when any element is not finite.
+// Sets *flag (mapped host memory) when any element is not finite.
 __global__ void heom_check_finite(const double* __restrict__ y, int64_t len, int* flag)
 {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     int bad = 0;
     for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < len; e += stride)
         bad |= !isfinite(y[e]);
-    if (__syncthreads_or(bad) && threadIdx.x == 0) atomicExch(flag, 1);
+    if (__syncthreads_or(bad) && threadIdx.x == 0) *static_cast<volatile int*>(flag) = 1;
 }
 
 } // namespace heomk

@@ -93,6 +93,27 @@ struct DevBuf {
     }
 };
 
+// a flag that kernels set and the host reads after the stream has drained: mapped pinned memory, so that a call that
+// checks it needs no copy of its own
+struct HostFlag {
+    int* host = nullptr;
+    int* dev = nullptr;
+    ~HostFlag()
+    {
+        if (host) cudaFreeHost(host);
+    }
+    int alloc()
+    {
+        cudaError_t e = cudaHostAlloc(&host, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable);
+        if (e == cudaSuccess) e = cudaHostGetDevicePointer(&dev, host, 0);
+        if (e != cudaSuccess) return fail(HEOM_E_NOMEM, "mapped flag: %s", cudaGetErrorString(e));
+        clear();
+        return 0;
+    }
+    void clear() { *static_cast<volatile int*>(host) = 0; }
+    bool set() const { return *static_cast<volatile int*>(host) != 0; }
+};
+
 typedef void (*dmma_fn_t)(const heomk::DmmaParams);
 typedef dmma_fn_t stage_fn_t;
 
@@ -256,6 +277,7 @@ struct heom_handle {
     int P = 0;          // 32-byte sectors per ADO (pair layout)
     int NW = 0, TWB = 0; // padded widths of the neighbour and tuple rows
     int hkind = heomk::H_REAL_SYM;
+    bool same_real = false; // pf_same and pf_same_sum are real (no bath with omega != 0)
 
     // instances: ADOs [inst_base[k], inst_base[k+1]) in both the reference
     // and the internal order belong to instance k
@@ -286,7 +308,7 @@ struct heom_handle {
     std::vector<int16_t> pair_tab;   // host copy
     heomk::RowTab row_tab{};         // sector positions of the N <= 8 stage kernel's lanes
     heomk::LaneTab lane_tab{};       // lane tables of the lockstep kernel
-    DevBuf<int> d_err;               // set by a stage kernel whose pipeline wait expired
+    HostFlag err;                    // set by a stage kernel whose pipeline wait expired
 
     // propagation state + stage buffers
     heom_buffer y;
@@ -295,7 +317,7 @@ struct heom_handle {
     int64_t xfer_ados = 0;
     DevBuf<double2> toplog;
     DevBuf<double2> topbuf; // row-major top matrices of all instances
-    DevBuf<int> d_flag;
+    HostFlag flag;                   // set by heom_check_finite
 
     // launch accounting and shape
     int64_t launches = 0;
@@ -524,6 +546,7 @@ PairParams base_params(const heom_handle* h)
     p.TWB = h->TWB;
     p.LS = h->LS;
     p.SL = h->SL;
+    p.same_real = h->same_real ? 1 : 0;
     return p;
 }
 
@@ -664,7 +687,7 @@ int launch_stage(heom_handle* h, int epi, const double2* in, const double2* y, d
     dp.ct.khat = adj && adj->khat ? adj->khat : h->d_khat.p;
     dp.ct.sq = h->d_sq.p;
     dp.ct.pos = h->d_pos.p;
-    dp.err = h->d_err.p;
+    dp.err = h->err.dev;
     if (h->kp) {
         // lockstep: every instance uses instance 0's rows of the shared tables
         heomk::LockParams lp;
@@ -1268,13 +1291,11 @@ int noalloc_scratch(int device, unsigned char** out)
     return 0;
 }
 
-// a stage kernel whose bounded pipeline wait expired leaves a flag behind
+// a stage kernel whose bounded pipeline wait expired leaves a flag behind (the handle's launches have drained)
 int check_kernel_error(heom_handle* h)
 {
-    int err = 0;
-    CUDA_TRY(cudaMemcpy(&err, h->d_err.p, sizeof(int), cudaMemcpyDeviceToHost));
-    if (err) {
-        cudaMemset(h->d_err.p, 0, sizeof(int));
+    if (h->err.set()) {
+        h->err.clear();
         return fail(HEOM_E_CUDA, "stage kernel pipeline wait expired (results of this call are invalid)");
     }
     return 0;
@@ -1421,6 +1442,9 @@ int heom_create_batch(const heom_instance_desc* descs, int32_t count, const heom
         std::copy(e->hamiltonian, e->hamiltonian + 2 * h->N * h->N, h->ham.begin() + (size_t)k * 2 * h->N * h->N);
     }
     h->mask.assign(h->nodes, 1);
+    h->same_real = true;
+    for (int b = 0; b < h->B; ++b) h->same_real = h->same_real && h->pf_same[2 * b + 1] == 0.0;
+    for (int64_t r = 0; r < h->nodes; ++r) h->same_real = h->same_real && h->pss[2 * r + 1] == 0.0;
     for (int q = 0; q < h->B * h->M; ++q)
         if (!(std::hypot(h->cbk[2 * q], h->cbk[2 * q + 1]) > 0.0))
             return fail(HEOM_E_TABLE, "cbk[%d] is zero or not finite", q);
@@ -1445,9 +1469,8 @@ int heom_create_batch(const heom_instance_desc* descs, int32_t count, const heom
     h->xfer_ados = std::max<int64_t>(1, std::min<int64_t>(h->nodes, (int64_t(64) << 20) / (nn * 16)));
     if (int rc = h->xfer.alloc((size_t)h->xfer_ados * nn)) return rc;
     if (int rc = h->topbuf.alloc((size_t)count * nn)) return rc;
-    if (int rc = h->d_flag.alloc(1)) return rc;
-    if (int rc = h->d_err.alloc(1)) return rc;
-    CUDA_TRY(cudaMemset(h->d_err.p, 0, sizeof(int)));
+    if (int rc = h->flag.alloc()) return rc;
+    if (int rc = h->err.alloc()) return rc;
     *out = h.release();
     return 0;
 }
@@ -1935,18 +1958,16 @@ int heom_propagate(heom_handle* h, double dt, int64_t steps, int64_t observe_eve
         h->launches++;
         CUDA_TRY(cudaGetLastError());
     }
+    // failure detection: a non-finite state is reported instead of returned silently
+    h->flag.clear();
+    heomk::heom_check_finite<<<h->sm_count * 4, 256, 0, h->stream>>>(
+        reinterpret_cast<const double*>(h->y.data.p), (int64_t)h->state_elems() * 2, h->flag.dev);
+    h->launches++;
+    CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaMemcpyAsync(host_tops, h->toplog.p, rows * nn * 16, cudaMemcpyDeviceToHost, h->stream));
     CUDA_TRY(cudaStreamSynchronize(h->stream));
-    // failure detection: a non-finite state is reported instead of returned silently
-    CUDA_TRY(cudaMemsetAsync(h->d_flag.p, 0, sizeof(int), h->stream));
-    heomk::heom_check_finite<<<h->sm_count * 4, 256, 0, h->stream>>>(
-        reinterpret_cast<const double*>(h->y.data.p), (int64_t)h->state_elems() * 2, h->d_flag.p);
-    h->launches++;
-    int flag = 0;
-    CUDA_TRY(cudaMemcpyAsync(&flag, h->d_flag.p, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-    CUDA_TRY(cudaStreamSynchronize(h->stream));
     if (int rc = check_kernel_error(h)) return rc;
-    if (flag) return fail(HEOM_E_NONFINITE, "non-finite value in the hierarchy state after propagation");
+    if (h->flag.set()) return fail(HEOM_E_NONFINITE, "non-finite value in the hierarchy state after propagation");
     return 0;
 }
 
@@ -2563,9 +2584,9 @@ int heom_ensemble_propagate(heom_ensemble* e, double dt, int64_t steps, int64_t 
     }
     // failure detection: a non-finite state is reported instead of returned silently
     for (heom_handle* h : e->cls) {
-        CUDA_TRY(cudaMemsetAsync(h->d_flag.p, 0, sizeof(int), e->stream));
+        h->flag.clear();
         heomk::heom_check_finite<<<h->sm_count * 4, 256, 0, e->stream>>>(
-            reinterpret_cast<const double*>(h->y.data.p), (int64_t)h->state_elems() * 2, h->d_flag.p);
+            reinterpret_cast<const double*>(h->y.data.p), (int64_t)h->state_elems() * 2, h->flag.dev);
         h->launches++;
         CUDA_TRY(cudaGetLastError());
     }
@@ -2579,9 +2600,7 @@ int heom_ensemble_propagate(heom_ensemble* e, double dt, int64_t steps, int64_t 
     }
     for (heom_handle* h : e->cls) {
         if (int rc = check_kernel_error(h)) return rc;
-        int flag = 0;
-        CUDA_TRY(cudaMemcpy(&flag, h->d_flag.p, sizeof(int), cudaMemcpyDeviceToHost));
-        if (flag) return fail(HEOM_E_NONFINITE, "non-finite value in the hierarchy state after propagation");
+        if (h->flag.set()) return fail(HEOM_E_NONFINITE, "non-finite value in the hierarchy state after propagation");
     }
     return 0;
 }
