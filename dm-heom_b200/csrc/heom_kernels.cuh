@@ -225,8 +225,8 @@ __device__ __forceinline__ void cmac(double2& acc, const double2 a, const double
 // cycles per ADO and SM; 88 of them shared memory) and the latency of 20 warps
 // per SM.  Measured against a lane per sector, which looked up both sites'
 // slots for two elements (us per stage, one B200): 8 states, two slots, 735,471
-// ADOs 791 -> 547, 74,613 ADOs 76.0 -> 51.8; one slot, 24,310 ADOs 21.5 -> 15.9,
-// 319,770 ADOs 235 -> 200; 7 states, one slot, 6435 ADOs 9.75 -> 6.7; 330 ADOs
+// ADOs 791 -> 547, 74,613 ADOs 76.0 -> 51.8; one slot, 24,310 ADOs 21.5 -> 14.9,
+// 319,770 ADOs 235 -> 217; 7 states, one slot, 6435 ADOs 9.75 -> 6.6; 330 ADOs
 // 4.6 -> 3.1 (mostly the dependent launch).  503 -> 347 instructions and 204 ->
 // 143 wavefronts per ADO; 47 of the 61 fewer are shared memory's, the rest a
 // store that is linear in the lanes (22 -> 8) and owned sectors side by side.
@@ -407,9 +407,11 @@ __device__ __forceinline__ int opaque(int v)
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 
-// CTAs of four warps per SM: five (96 registers a thread, 20 warps) where that does not spill (8 states, two
-// slots, 735,471 ADOs: 547 us a stage, against 608 at 16 warps and 789 at 24 with 56 bytes spilled)
-constexpr int row_blocks(int hk, int slt, bool mi) { return hk == H_REAL_SYM && slt <= 2 && !mi ? 5 : 4; }
+// CTAs of four warps per SM. Two slots: five (96 registers a thread, 20 warps; 8 states, 735,471 ADOs: 547 us a
+// stage, against 608 at 16 warps and 789 at 24 with 56 bytes spilled). One slot: four (8 states, 24,310 ADOs 14.9
+// us, 7 states, 6435 ADOs 6.6; five spill a little: 15.4 and 7.0, and gain only far beyond L2, 319,770 ADOs 211 us
+// against 217). Complex H, batches and more slots need the registers.
+constexpr int row_blocks(int hk, int slt, bool mi) { return hk == H_REAL_SYM && slt == 2 && !mi ? 5 : 4; }
 
 // MI: the handle holds several instances (p.inst set); each ADO's instance
 // selects its H fragments, reloaded whenever the instance changes.
@@ -1253,7 +1255,11 @@ __global__ void heom_write_top(double2* __restrict__ y, const double2* __restric
 //   lambda, gamma (shared by all baths): L is linear in its coefficient
 //           tables, so dL/dtheta is L with H = 0 and the tables replaced by
 //           their derivatives (dpss, dgamma0, dchat, dkhat).
-// One warp per ADO; lanes own sectors (pair layout).  The blocks are split
+// One warp per ADO; its lanes take the (state, column pair) threads of the
+// stage kernels in turn, so that the look-ups of a slot serve four elements, and
+// the derivative tables lie in shared memory.  Latency bounds it: 4 instances of
+// 9 states, 715 ADOs each, 18 us a factor with a lane per sector and its tables
+// in global memory.  The blocks are split
 // among the instances of the handle (each block sweeps one instance's ADOs),
 // and every block adds weight * (its sum) to its own row of `partial`
 // (deterministic; summed per instance on the host at the end).
@@ -1278,25 +1284,66 @@ struct GradParams {
     double2* partial;                  // [gridDim.x][N*N + 2]
     const int64_t* inst_base;          // [instances + 1] first ADO of every instance
     int blocks_per_inst;               // blocks [k*bpi, (k+1)*bpi) sweep instance k only
-    int N, P, W, NW, TWB, SL;
+    int N, P, W, NW, TWB, SL, LS;
     int want_h;                        // accumulate Z (the H gradient)
     int want_bath;                     // accumulate <a, L_theta' w> (the lambda and gamma gradients)
 };
 
+// one (state, column pair) of heom_adjoint_grad, as a lane of the stage kernels: its owned and handed-over sector
+// (-1: none), the elements of the owned one, tile positions of its halves and of the other's row and column element
+struct GradLane {
+    short r, diag, pso, psg, e1, e2, q1, q2, gr, gc, twin, pad; // diag 1: the owned sector is diagonal, 2: the other
+};
 __host__ __device__ inline int grad_warp_bytes(int n) { return 2 * n * (n + 1) * 16; }
-__host__ inline size_t grad_smem_bytes(int n)
+__host__ inline size_t grad_smem_bytes(int n, int W, int LS)
 {
-    return (size_t)kCtaWarps * grad_warp_bytes(n) + (size_t)(kCtaWarps + 1) * (n * n + 2) * 16;
+    return (size_t)kCtaWarps * grad_warp_bytes(n) + (size_t)(kCtaWarps + 1) * (n * n + 2) * 16 +
+           (size_t)(2 * n * n + 5 * W) * 16 + (size_t)((LS + 2) & ~1) * 8 + (size_t)n * ((n + 1) / 2) * sizeof(GradLane);
 }
 
 __global__ void __launch_bounds__(kCtaWarps * 32) heom_adjoint_grad(const __grid_constant__ GradParams g)
 {
     extern __shared__ __align__(128) unsigned char smem[];
-    const int N = g.N, P = g.P, W = g.W, SL = g.SL, NN = N * N;
+    const int N = g.N, P = g.P, W = g.W, SL = g.SL, NN = N * N, LD = N + 1;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     double2* At = reinterpret_cast<double2*>(smem + warp * grad_warp_bytes(N)); // [N][N+1]
-    double2* Wt = At + N * (N + 1);
+    double2* Wt = At + N * LD;
     double2* red = reinterpret_cast<double2*>(smem + kCtaWarps * grad_warp_bytes(N)); // [warps][NN+2]
+    double2* acc = red + kCtaWarps * (NN + 2);                                         // [NN+2]
+    // derivative tables, lambda and gamma side by side: dg0 [NN][2], dkhat side i and side j [W][4], dchat [W]
+    double2* s_dg = acc + NN + 2;
+    double2* s_dk = s_dg + 2 * NN;
+    double2* s_dc = s_dk + 4 * W;
+    double* s_sq = reinterpret_cast<double*>(s_dc + W);                                // [LS+1]
+    GradLane* lanes = reinterpret_cast<GradLane*>(s_sq + ((g.LS + 2) & ~1));           // [N T]
+    for (int q = threadIdx.x; q < 2 * NN; q += blockDim.x) s_dg[q] = g.dg0[(q & 1) * NN + (q >> 1)];
+    for (int q = threadIdx.x; q < 4 * W; q += blockDim.x) s_dk[q] = g.dkhat[(q & 1) * 3 * W + ((q >> 1) & 1) * W + (q >> 2)];
+    for (int q = threadIdx.x; q < W; q += blockDim.x) s_dc[q] = make_double2(g.dchat[q], g.dchat[W + q]);
+    for (int q = threadIdx.x; q <= g.LS; q += blockDim.x) s_sq[q] = g.sq[q];
+    const int T = (N + 1) / 2, NL = N * T;
+    for (int l = threadIdx.x; l < NL; l += blockDim.x) {
+        const int r = l / T, t = l - r * T, R = r >> 1, odd = row_owned(r, t);
+        const int co = 2 * t + odd, cg = 2 * t + 1 - odd;
+        const bool dga = t == R && !(r & 1), dgb = t == R && (r & 1);
+        GradLane q;
+        q.r = r;
+        q.diag = dga ? 1 : dgb ? 2 : 0;
+        q.pso = q.psg = -1;
+        for (int p = 0; p < P; ++p) { // the sectors that hold (r, co) and (r, cg)
+            const int e1 = g.pe[2 * p], e2 = g.pe[2 * p + 1];
+            if (co < N && (e1 == r * N + co || e2 == r * N + co)) q.pso = p;
+            if (cg < N && (e1 == r * N + cg || e2 == r * N + cg)) q.psg = p;
+        }
+        const int i2 = dga ? (r + 1 < N ? r + 1 : r) : co, j2 = dga ? i2 : r;
+        q.twin = dga && i2 == r;
+        q.e1 = co < N ? r * N + co : 0;
+        q.e2 = co < N ? i2 * N + j2 : 0;
+        q.q1 = co < N ? r * LD + co : 0;
+        q.q2 = co < N ? i2 * LD + j2 : 0;
+        q.gr = cg < N ? r * LD + cg : 0;
+        q.gc = cg < N ? (dgb ? q.gr : cg * LD + r) : 0;
+        lanes[l] = q;
+    }
     // Z on the FP64 tensor pipe: blocks (I, J) of 8 x 8 of the zero-padded Z (one block for
     // N <= 8, 2 x 2 for N <= 16), accumulated over the warp's ADOs in the MMA fragments:
     // lane 4g + t holds Z(8I+g, 8J+2t) and Z(8I+g, 8J+2t+1), real and imaginary parts
@@ -1304,159 +1351,173 @@ __global__ void __launch_bounds__(kCtaWarps * 32) heom_adjoint_grad(const __grid
     const int nblk = N <= 8 ? 1 : 4, ks = (N + 3) / 4;
     double zr[4][2], zi[4][2];
     auto el = [&](const double2* T, int r, int c) {
-        return (r < N && c < N) ? T[r * (N + 1) + c] : make_double2(0.0, 0.0);
+        return (r < N && c < N) ? T[r * LD + c] : make_double2(0.0, 0.0);
+    };
+    auto conj_mac = [](double2& s, const double2 a, const double2 w) { // s += conj(a) w
+        s.x = fma(a.x, w.x, s.x);
+        s.x = fma(a.y, w.y, s.x);
+        s.y = fma(a.x, w.y, s.y);
+        s.y = fma(-a.y, w.x, s.y);
     };
 
     const int inst = blockIdx.x / g.blocks_per_inst, jb = blockIdx.x - inst * g.blocks_per_inst;
     const int64_t stride = (int64_t)g.blocks_per_inst * kCtaWarps, end = g.inst_base[inst + 1];
-    double2* acc = red + kCtaWarps * (NN + 2); // [NN+2]
     double2* const out = g.partial + (int64_t)blockIdx.x * (NN + 2);
     for (int q = threadIdx.x; q < NN + 2; q += blockDim.x) acc[q] = out[q];
+    __syncthreads();
     for (int f = 0; f < g.factors; ++f) {
-    const double2* a_in = g.a + f * g.a_step;
-    const double2* w_in = g.w + f * g.w_step;
+        const double2* a_in = g.a + f * g.a_step;
+        const double2* w_in = g.w + f * g.w_step;
+        const double2 z0 = make_double2(0.0, 0.0);
 #pragma unroll
-    for (int b = 0; b < 4; ++b) zr[b][0] = zr[b][1] = zi[b][0] = zi[b][1] = 0.0;
-    double2 dl = make_double2(0.0, 0.0), dgm = dl;
-    for (int64_t u = g.inst_base[inst] + (int64_t)jb * kCtaWarps + warp; u < end; u += stride) {
-        const unsigned char* nb = g.rec + u * rec_bytes(g.NW, g.TWB);
-        const unsigned char* tu = nb + g.NW * 4;
-        const double dps = g.dpss[u];
-        for (int p = lane; p < P; p += 32) {
-            const int e1 = g.pe[2 * p], e2 = g.pe[2 * p + 1];
-            const int i1 = e1 / N, j1 = e1 - i1 * N, i2 = e2 / N, j2 = e2 - i2 * N;
-            double2 a1, a2, w1, w2;
-            ld256(a_in + (u * P + p) * 2, a1, a2);
-            ld256(w_in + (u * P + p) * 2, w1, w2);
-            At[i1 * (N + 1) + j1] = a1;
-            At[i2 * (N + 1) + j2] = a2;
-            Wt[i1 * (N + 1) + j1] = w1;
-            Wt[i2 * (N + 1) + j2] = w2;
-            const bool diag = i1 == j1;
-            const bool twin = e2 == e1; // padding half of an odd diagonal pair
-            if (!g.want_bath) continue;
-            // derivative of the operator applied to w, for theta = lambda (0), gamma (1)
-            double2 D1[2], D2[2];
-            for (int th = 0; th < 2; ++th) {
-                const double2 s1 = g.dg0[th * NN + e1], s2 = g.dg0[th * NN + e2];
-                const double sp = th == 1 ? dps : 0.0;
-                D1[th] = make_double2((sp + s1.x) * w1.x - s1.y * w1.y, (sp + s1.x) * w1.y + s1.y * w1.x);
-                D2[th] = make_double2((sp + s2.x) * w2.x - s2.y * w2.y, (sp + s2.x) * w2.y + s2.y * w2.x);
+        for (int b = 0; b < 4; ++b) zr[b][0] = zr[b][1] = zi[b][0] = zi[b][1] = 0.0;
+        double2 dl = z0, dgm = z0;
+        for (int64_t u = g.inst_base[inst] + (int64_t)jb * kCtaWarps + warp; u < end; u += stride) {
+            const unsigned char* nb = g.rec + u * rec_bytes(g.NW, g.TWB);
+            const unsigned char* tu = nb + g.NW * 4;
+            const double dps = g.dpss[u];
+            for (int l = lane; l < NL; l += 32) {
+                const GradLane q = lanes[l];
+                if (q.pso < 0) continue;
+                double2 a1, a2, w1, w2;
+                ld256_cg(a_in + (u * P + q.pso) * 2, a1, a2);
+                ld256_cg(w_in + (u * P + q.pso) * 2, w1, w2);
+                At[q.q1] = a1;
+                At[q.q2] = a2;
+                Wt[q.q1] = w1;
+                Wt[q.q2] = w2;
             }
-            // bath terms: side 0 = slots of site i1, side 1 = slots of site j1
-            // (diagonal pairs: element 1 takes the slots of i1, element 2 those of i2)
-            for (int sd = 0; sd < 2; ++sd) {
-                const int site = sd == 0 ? i1 : (diag ? i2 : j1);
-                for (int q = 0; q < SL; ++q) {
-                    const int sl = g.slots[site * SL + q];
-                    if (sl < 0) continue;
-                    const int n = tu[sl];
-                    const int2 pm = reinterpret_cast<const int2*>(nb)[sl];
-                    const int32_t vp = diag ? -1 : pm.x;
-                    const int32_t vm = pm.y;
-                    double2 p1 = make_double2(0.0, 0.0), p2 = p1, m1 = p1, m2 = p1;
-                    if (vp >= 0) ld256(w_in + ((int64_t)vp * P + p) * 2, p1, p2);
-                    if (vm >= 0) ld256(w_in + ((int64_t)vm * P + p) * 2, m1, m2);
-                    const double shi = g.sq[n + 1], slo = g.sq[n];
-                    for (int th = 0; th < 2; ++th) {
-                        const double c = g.dchat[th * W + sl] * shi;
-                        const double2* kh = g.dkhat + th * 3 * W;
-                        if (diag) {
-                            // element (site, site): kappa_i + kappa_j only
-                            const double2 k = kh[2 * W + sl];
-                            double2& D = sd == 0 ? D1[th] : D2[th];
-                            cmac(D, make_double2(k.x * slo, k.y * slo), sd == 0 ? m1 : m2);
-                        } else if (sd == 0) {
-                            // site i: element 1 (i,j) i-side, element 2 (j,i) j-side
-                            D1[th].x -= c * p1.y; D1[th].y += c * p1.x;
-                            D2[th].x += c * p2.y; D2[th].y -= c * p2.x;
-                            const double2 ki = kh[sl], kj = kh[W + sl];
-                            cmac(D1[th], make_double2(ki.x * slo, ki.y * slo), m1);
-                            cmac(D2[th], make_double2(kj.x * slo, kj.y * slo), m2);
-                        } else {
-                            D1[th].x += c * p1.y; D1[th].y -= c * p1.x;
-                            D2[th].x -= c * p2.y; D2[th].y += c * p2.x;
-                            const double2 ki = kh[sl], kj = kh[W + sl];
-                            cmac(D1[th], make_double2(kj.x * slo, kj.y * slo), m1);
-                            cmac(D2[th], make_double2(ki.x * slo, ki.y * slo), m2);
+            __syncwarp();
+            if (g.want_bath)
+                for (int l = lane; l < NL; l += 32) {
+                    const GradLane q = lanes[l];
+                    const double2 a1 = At[q.q1], a2 = At[q.q2], ar = At[q.gr], ac = At[q.gc];
+                    // same term of the owned elements (a padding half counts once)
+                    if (q.pso >= 0) {
+                        double2 v1 = z0, v2 = z0;
+                        conj_mac(v1, a1, Wt[q.q1]);
+                        if (!q.twin) conj_mac(v2, a2, Wt[q.q2]);
+                        cmac(dl, s_dg[2 * q.e1], v1);
+                        cmac(dl, s_dg[2 * q.e2], v2);
+                        const double2 s1 = s_dg[2 * q.e1 + 1], s2 = s_dg[2 * q.e2 + 1];
+                        cmac(dgm, make_double2(s1.x + dps, s1.y), v1);
+                        cmac(dgm, make_double2(s2.x + dps, s2.y), v2);
+                    }
+                    for (int k = 0; k < SL; ++k) {
+                        const int sl = g.slots[q.r * SL + k];
+                        if (sl < 0) continue;
+                        const int2 pm = __ldg(reinterpret_cast<const int2*>(nb) + sl);
+                        const int n = tu[sl];
+                        double2 mo[2], mg[2], po[2], pg[2]; // minus and plus neighbour, owned and handed-over sector
+                        const int no = q.pso < 0 ? -1 : 0, ng = q.psg < 0 ? -1 : 0;
+                        const int co = q.diag == 1 ? -1 : no, cg = q.diag == 2 ? -1 : ng; // plus terms of a diagonal cancel
+                        const double2* bo = w_in + (q.pso < 0 ? 0 : q.pso) * 2;
+                        const double2* bg = w_in + (q.psg < 0 ? 0 : q.psg) * 2;
+                        ld256_if(pm.y | no, bo + (int64_t)pm.y * (2 * P), mo[0], mo[1]);
+                        ld256_if(pm.y | ng, bg + (int64_t)pm.y * (2 * P), mg[0], mg[1]);
+                        ld256_if(pm.x | co, bo + (int64_t)pm.x * (2 * P), po[0], po[1]);
+                        ld256_if(pm.x | cg, bg + (int64_t)pm.x * (2 * P), pg[0], pg[1]);
+                        if (pm.y >= 0) {
+                            double2 vi = z0, vj = z0; // row and column elements
+                            if (no >= 0) {
+                                conj_mac(vi, a1, mo[0]);
+                                conj_mac(vj, q.diag == 1 ? a1 : a2, q.diag == 1 ? mo[0] : mo[1]);
+                            }
+                            if (ng >= 0) {
+                                conj_mac(vi, ar, mg[1]);
+                                conj_mac(vj, ac, q.diag == 2 ? mg[1] : mg[0]);
+                            }
+                            const double s = s_sq[n];
+                            vi = make_double2(vi.x * s, vi.y * s);
+                            vj = make_double2(vj.x * s, vj.y * s);
+                            const double2* dk = s_dk + 4 * sl;
+                            cmac(dl, dk[0], vi);
+                            cmac(dgm, dk[1], vi);
+                            cmac(dl, dk[2], vj);
+                            cmac(dgm, dk[3], vj);
+                        }
+                        if (pm.x >= 0) {
+                            double2 vr = z0, vc = z0; // row elements with +i, column elements with -i
+                            if (co >= 0) {
+                                conj_mac(vr, a1, po[0]);
+                                conj_mac(vc, a2, po[1]);
+                            }
+                            if (cg >= 0) {
+                                conj_mac(vr, ar, pg[1]);
+                                conj_mac(vc, ac, pg[0]);
+                            }
+                            const double s = s_sq[n + 1];
+                            const double vx = s * (vc.y - vr.y), vy = s * (vr.x - vc.x); // i (vr - vc)
+                            const double2 c = s_dc[sl];
+                            dl.x = fma(c.x, vx, dl.x);
+                            dl.y = fma(c.x, vy, dl.y);
+                            dgm.x = fma(c.y, vx, dgm.x);
+                            dgm.y = fma(c.y, vy, dgm.y);
                         }
                     }
                 }
-            }
-            // <a, D>: conj(a) * D over the sector's elements (a padding half counts once)
-            double2* acc[2] = {&dl, &dgm};
-            for (int th = 0; th < 2; ++th) {
-                acc[th]->x += a1.x * D1[th].x + a1.y * D1[th].y;
-                acc[th]->y += a1.x * D1[th].y - a1.y * D1[th].x;
-                if (!twin) {
-                    acc[th]->x += a2.x * D2[th].x + a2.y * D2[th].y;
-                    acc[th]->y += a2.x * D2[th].y - a2.y * D2[th].x;
+            // Z(k,l) = sum_i w(i,k) conj(a(i,l)) - sum_j conj(a(k,j)) w(l,j):
+            //   Re Z = Wr^T Ar + Wi^T Ai - Ar Wr^T - Ai Wi^T, Im Z = Wi^T Ar - Wr^T Ai - Ar Wi^T + Ai Wr^T
+            if (g.want_h) {
+#pragma unroll
+                for (int b = 0; b < 4; ++b) {
+                    if (b >= nblk) continue;
+                    const int I = b >> 1, J = b & 1;
+#pragma unroll
+                    for (int s = 0; s < 4; ++s) {
+                        if (s >= ks) continue;
+                        const int k0 = 4 * s + t4;
+                        const double2 wT = el(Wt, k0, 8 * I + gq); // A operand of W^T A: W(4s+t, 8I+g)
+                        const double2 aB = el(At, k0, 8 * J + gq); // B operand of W^T A: A(4s+t, 8J+g)
+                        const double2 aA = el(At, 8 * I + gq, k0); // A operand of A W^T: A(8I+g, 4s+t)
+                        const double2 wB = el(Wt, 8 * J + gq, k0); // B operand of A W^T: W(8J+g, 4s+t)
+                        dmma(zr[b][0], zr[b][1], wT.x, aB.x);
+                        dmma(zr[b][0], zr[b][1], wT.y, aB.y);
+                        dmma(zr[b][0], zr[b][1], -aA.x, wB.x);
+                        dmma(zr[b][0], zr[b][1], -aA.y, wB.y);
+                        dmma(zi[b][0], zi[b][1], wT.y, aB.x);
+                        dmma(zi[b][0], zi[b][1], -wT.x, aB.y);
+                        dmma(zi[b][0], zi[b][1], -aA.x, wB.y);
+                        dmma(zi[b][0], zi[b][1], aA.y, wB.x);
+                    }
                 }
             }
+            __syncwarp();
         }
-        __syncwarp();
-        // Z(k,l) = sum_i w(i,k) conj(a(i,l)) - sum_j conj(a(k,j)) w(l,j):
-        //   Re Z = Wr^T Ar + Wi^T Ai - Ar Wr^T - Ai Wi^T, Im Z = Wi^T Ar - Wr^T Ai - Ar Wi^T + Ai Wr^T
-        if (g.want_h) {
+        // block sum in a fixed order, then weight * sum into this block's row
+        double2* mine = red + warp * (NN + 2);
 #pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                if (b >= nblk) continue;
-                const int I = b >> 1, J = b & 1;
+        for (int b = 0; b < 4; ++b) {
+            if (b >= nblk) continue;
+            const int r = 8 * (b >> 1) + gq;
 #pragma unroll
-                for (int s = 0; s < 4; ++s) {
-                    if (s >= ks) continue;
-                    const int k0 = 4 * s + t4;
-                    const double2 wT = el(Wt, k0, 8 * I + gq); // A operand of W^T A: W(4s+t, 8I+g)
-                    const double2 aB = el(At, k0, 8 * J + gq); // B operand of W^T A: A(4s+t, 8J+g)
-                    const double2 aA = el(At, 8 * I + gq, k0); // A operand of A W^T: A(8I+g, 4s+t)
-                    const double2 wB = el(Wt, 8 * J + gq, k0); // B operand of A W^T: W(8J+g, 4s+t)
-                    dmma(zr[b][0], zr[b][1], wT.x, aB.x);
-                    dmma(zr[b][0], zr[b][1], wT.y, aB.y);
-                    dmma(zr[b][0], zr[b][1], -aA.x, wB.x);
-                    dmma(zr[b][0], zr[b][1], -aA.y, wB.y);
-                    dmma(zi[b][0], zi[b][1], wT.y, aB.x);
-                    dmma(zi[b][0], zi[b][1], -wT.x, aB.y);
-                    dmma(zi[b][0], zi[b][1], -aA.x, wB.y);
-                    dmma(zi[b][0], zi[b][1], aA.y, wB.x);
-                }
+            for (int e = 0; e < 2; ++e) {
+                const int c = 8 * (b & 1) + 2 * t4 + e;
+                if (r < N && c < N) mine[r * N + c] = make_double2(zr[b][e], zi[b][e]);
             }
         }
-        __syncwarp();
-    }
-    // block sum in a fixed order, then weight * sum into this block's row
-    double2* mine = red + warp * (NN + 2);
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-        if (b >= nblk) continue;
-        const int r = 8 * (b >> 1) + gq;
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            const int c = 8 * (b & 1) + 2 * t4 + e;
-            if (r < N && c < N) mine[r * N + c] = make_double2(zr[b][e], zi[b][e]);
+        for (int off = 16; off > 0; off >>= 1) {
+            dl.x += __shfl_down_sync(0xffffffffu, dl.x, off);
+            dl.y += __shfl_down_sync(0xffffffffu, dl.y, off);
+            dgm.x += __shfl_down_sync(0xffffffffu, dgm.x, off);
+            dgm.y += __shfl_down_sync(0xffffffffu, dgm.y, off);
         }
-    }
-    for (int off = 16; off > 0; off >>= 1) {
-        dl.x += __shfl_down_sync(0xffffffffu, dl.x, off);
-        dl.y += __shfl_down_sync(0xffffffffu, dl.y, off);
-        dgm.x += __shfl_down_sync(0xffffffffu, dgm.x, off);
-        dgm.y += __shfl_down_sync(0xffffffffu, dgm.y, off);
-    }
-    if (lane == 0) {
-        mine[NN] = dl;
-        mine[NN + 1] = dgm;
-    }
-    __syncthreads();
-    for (int q = threadIdx.x; q < NN + 2; q += blockDim.x) {
-        double2 s = make_double2(0.0, 0.0);
-        for (int v = 0; v < kCtaWarps; ++v) {
-            s.x += red[v * (NN + 2) + q].x;
-            s.y += red[v * (NN + 2) + q].y;
+        if (lane == 0) {
+            mine[NN] = dl;
+            mine[NN + 1] = dgm;
         }
+        __syncthreads();
         const double2 wgt = g.weight[(g.factor0 - f) & 3];
-        acc[q].x += wgt.x * s.x - wgt.y * s.y;
-        acc[q].y += wgt.x * s.y + wgt.y * s.x;
-    }
-    __syncthreads();
+        for (int q = threadIdx.x; q < NN + 2; q += blockDim.x) {
+            double2 s = z0;
+            for (int v = 0; v < kCtaWarps; ++v) {
+                s.x += red[v * (NN + 2) + q].x;
+                s.y += red[v * (NN + 2) + q].y;
+            }
+            acc[q].x += wgt.x * s.x - wgt.y * s.y;
+            acc[q].y += wgt.x * s.y + wgt.y * s.x;
+        }
+        __syncthreads();
     }
     for (int q = threadIdx.x; q < NN + 2; q += blockDim.x) out[q] = acc[q];
 }

@@ -93,25 +93,65 @@ struct DevBuf {
     }
 };
 
-// a flag that kernels set and the host reads after the stream has drained: mapped pinned memory, so that a call that
-// checks it needs no copy of its own
-struct HostFlag {
+// Flags that kernels set and the host reads after the stream has drained: mapped pinned memory, so that a call that
+// checks one needs no copy of its own.  Page-locking takes longer than the rest of a small handle's creation, so the
+// handles share a page of flags, which goes with the last of them.
+struct FlagPage {
+    static constexpr int kFlags = 1024;
     int* host = nullptr;
-    int* dev = nullptr;
-    ~HostFlag()
+    std::vector<int> unused;
+    std::mutex mu;
+    ~FlagPage()
     {
         if (host) cudaFreeHost(host);
     }
+};
+std::mutex g_flag_mu;
+std::weak_ptr<FlagPage> g_flag_page; // the page that new flags come from
+
+struct HostFlag {
+    std::shared_ptr<FlagPage> page;
+    int index = -1;
+    int* dev = nullptr;
+    ~HostFlag()
+    {
+        if (!page) return;
+        std::lock_guard<std::mutex> lock(page->mu);
+        page->unused.push_back(index);
+    }
     int alloc()
     {
-        cudaError_t e = cudaHostAlloc(&host, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable);
-        if (e == cudaSuccess) e = cudaHostGetDevicePointer(&dev, host, 0);
-        if (e != cudaSuccess) return fail(HEOM_E_NOMEM, "mapped flag: %s", cudaGetErrorString(e));
+        std::lock_guard<std::mutex> lock(g_flag_mu);
+        std::shared_ptr<FlagPage> pg = g_flag_page.lock();
+        bool full = !pg;
+        if (pg) {
+            std::lock_guard<std::mutex> pl(pg->mu);
+            full = pg->unused.empty();
+        }
+        if (full) {
+            pg = std::make_shared<FlagPage>();
+            const cudaError_t e =
+                cudaHostAlloc(&pg->host, FlagPage::kFlags * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable);
+            if (e != cudaSuccess) {
+                pg->host = nullptr;
+                return fail(HEOM_E_NOMEM, "mapped flags: %s", cudaGetErrorString(e));
+            }
+            for (int q = FlagPage::kFlags - 1; q >= 0; --q) pg->unused.push_back(q);
+            g_flag_page = pg;
+        }
+        int* base = nullptr; // this device's address of the page
+        const cudaError_t e = cudaHostGetDevicePointer(&base, pg->host, 0);
+        if (e != cudaSuccess) return fail(HEOM_E_CUDA, "mapped flags: %s", cudaGetErrorString(e));
+        std::lock_guard<std::mutex> pl(pg->mu);
+        index = pg->unused.back();
+        pg->unused.pop_back();
+        page = pg;
+        dev = base + index;
         clear();
         return 0;
     }
-    void clear() { *static_cast<volatile int*>(host) = 0; }
-    bool set() const { return *static_cast<volatile int*>(host) != 0; }
+    void clear() { static_cast<volatile int*>(page->host)[index] = 0; }
+    bool set() const { return static_cast<volatile int*>(page->host)[index] != 0; }
 };
 
 typedef void (*dmma_fn_t)(const heomk::DmmaParams);
@@ -945,6 +985,7 @@ int run_steps(heom_handle* h, double dt, int64_t steps)
         // make sure launch shapes are resolved outside of capture
         const void* fn = nullptr;
         if (int rc = resolve_stage(h, &fn)) return rc;
+        if (int rc = resolve_stage(h, &fn, nullptr, false, true)) return rc;
         cudaGraph_t graph = nullptr;
         const int64_t saved = h->launches;
         CUDA_TRY(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
@@ -2351,6 +2392,7 @@ int ens_run_steps(heom_ensemble* e, double dt, int64_t steps)
         if (int rc = prepare_scheme(h)) return rc;
         const void* fn = nullptr;
         if (int rc = resolve_stage(h, &fn)) return rc;
+        if (int rc = resolve_stage(h, &fn, nullptr, false, true)) return rc;
         if (h->stage_smem == 0) return fail(HEOM_E_CUDA, "stage kernel shape unresolved");
     }
     if (!e->opt.use_graphs) {
@@ -2801,6 +2843,7 @@ int adj_grad(heom_adjoint* A, const double2* a, const double2* w, double dt, int
     g.NW = h->NW;
     g.TWB = h->TWB;
     g.SL = h->SL;
+    g.LS = h->LS;
     g.want_h = A->want_h;
     g.want_bath = A->want_bath;
     pick_grad(h->N, h->SL)<<<A->grid, heomk::kCtaWarps * 32, A->grad_smem, h->stream>>>(g);
@@ -3092,7 +3135,7 @@ int heom_adjoint_create_batch(const heom_system_desc* systems, int32_t count, co
     if (int rc = A->partial.alloc((size_t)A->grid * (h->N * h->N + 2))) return rc;
     if (int rc = A->inst_base.alloc(count + 1)) return rc;
     CUDA_TRY(cudaMemcpy(A->inst_base.p, h->inst_base.data(), (count + 1) * 8, cudaMemcpyHostToDevice));
-    A->grad_smem = heomk::grad_smem_bytes(h->N);
+    A->grad_smem = heomk::grad_smem_bytes(h->N, h->W, h->LS);
     if (int rc = allow_dynamic_smem((const void*)pick_grad(h->N, h->SL), A->grad_smem)) return rc;
     *out = A.release();
     return 0;
@@ -3128,8 +3171,13 @@ int heom_adjoint_gradient(heom_adjoint* A, const double* rho0, const double* obs
     // without a limit a slack stays free for the sweep's small buffers (top
     // log, weights, graphs) and the allocator's granularity.
     if (int rc = prepare_scheme(h)) return rc;
-    int64_t slots = 0;
-    {
+    // Small hierarchies: the gradient launches of a few steps are one, over a ring of adjoint states of at most
+    // kRingBytes. A launch over 6435 ADOs leaves a warp three of them and is prologue, tail and latency (7 sites, depth
+    // 8: 17 us a factor alone); from 16 MB a state a launch fills the device by itself. The ring takes no room from the
+    // checkpoints.
+    int64_t slots = 0, group = A->mem_limit == 0 ? std::min<int64_t>(S, (int64_t)(kRingBytes / (4 * st * 16))) : 0;
+    // (free memory, whose query can take a millisecond, is of no interest while the last call's buffers do)
+    if (A->mem_limit != 0 || !A->ga.p || ncp > A->cap_cps || 4 * S > A->cap_seg || 4 * (size_t)group * st > A->ring.n) {
         size_t free_b = 0, total_b = 0;
         CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
         const double sb = (double)st * 16.0;
@@ -3145,20 +3193,11 @@ int heom_adjoint_gradient(heom_adjoint* A, const double* rho0, const double* obs
             S = 1;
             ncp = slots;
         }
+        if (slots > 0 || (A->ring.n < 4 * (size_t)group * st &&
+                          (double)free_b < (double)(ncp + 4 * S + 3) * sb + 2.0 * kRingBytes))
+            group = 0;
     }
     A->rec_slots = slots;
-    // Small hierarchies: the gradient launches of a few steps are one, over a ring of adjoint states of at most
-    // kRingBytes. A launch over 6435 ADOs leaves a warp three of them and is prologue, tail and latency (7 sites, depth
-    // 8: 17 us a factor alone); from 16 MB a state a launch fills the device by itself. The ring takes no room from the
-    // checkpoints.
-    int64_t group = 0;
-    if (slots == 0 && A->mem_limit == 0) {
-        const size_t sb = st * 16;
-        group = std::min<int64_t>(S, (int64_t)(kRingBytes / (4 * sb)));
-        size_t free_b = 0, total_b = 0;
-        CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
-        if (A->ring.n < 4 * (size_t)group * st && free_b < (size_t)(ncp + 4 * S + 3) * sb + 2 * kRingBytes) group = 0;
-    }
     if (group != A->group) {
         A->drop_graphs();
         A->group = group;
