@@ -218,8 +218,9 @@ __device__ __forceinline__ void cmac(double2& acc, const double2 a, const double
 //
 // Pipeline: per warp two slots, each filled by two 1-D TMA bulk copies (tile,
 // record) that complete on the slot's mbarrier; the copies of ADO k+1 fly
-// while ADO k is computed.  Every wait is bounded; on expiry the kernel sets
-// *p.err and the warp stops.
+// while ADO k is computed.  Every wait is bounded and ends the same for all
+// lanes of the warp; on expiry the warp waits (bounded again) for the copies it
+// has in flight, sets *err and leaves as a whole.
 //
 // What bounds it: the L1 data pipe (8 states, two slots: 143 wavefronts of 194
 // cycles per ADO and SM; 88 of them shared memory) and the latency of 20 warps
@@ -346,11 +347,16 @@ __device__ __forceinline__ void mbar_expect(uint64_t* bar, unsigned bytes)
                  : "memory");
 }
 
+// tries of a bounded wait; an expression, so that a test can let the waits of chosen lanes run out
+#ifndef HEOM_WAIT_TRIES
+#define HEOM_WAIT_TRIES (1 << 24)
+#endif
+
 // bounded wait for the phase `parity` of an mbarrier; false on expiry
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity)
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity, int tries)
 {
     const unsigned a = smem_addr(bar);
-    for (int it = 0; it < (1 << 24); ++it) {
+    for (int it = 0; it < tries; ++it) {
         unsigned done;
         asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
                      " selp.u32 %0, 1, 0, p;\n}\n"
@@ -576,11 +582,16 @@ __global__ void __launch_bounds__(kRowWarps * 32, row_blocks(HK, SLT, MI)) heom_
         }
     };
     unsigned it = 0; // ADOs done: slot it & 1, mbarrier parity (it >> 1) & 1
+    // whether the copies of the warp's k-th ADO have arrived: the same for every lane, since what follows is the whole
+    // warp's work (MMAs, shuffles) and a warp gives up as a whole
+    auto arrived = [&](unsigned k) {
+        return __all_sync(0xffffffffu, mbar_wait(bars + (k & 1), (k >> 1) & 1, HEOM_WAIT_TRIES)) != 0;
+    };
     bool failed = false;
     if (u < nodes) {
         if (lane == 0) issue(u, slot, bars);
         if (AHEAD) {
-            if (mbar_wait(bars, 0)) load_k(slot, 0);
+            if (arrived(0)) load_k(slot, 0);
             else failed = true;
         }
     }
@@ -597,7 +608,7 @@ __global__ void __launch_bounds__(kRowWarps * 32, row_blocks(HK, SLT, MI)) heom_
             ni_ahead = u + 2 * stride < nodes ? __ldg(p.inst + u + 2 * stride) : ni;
         }
         if (!AHEAD) {
-            if (!mbar_wait(bars + (it & 1), (it >> 1) & 1)) {
+            if (!arrived(it)) {
                 failed = true;
                 break;
             }
@@ -718,7 +729,7 @@ __global__ void __launch_bounds__(kRowWarps * 32, row_blocks(HK, SLT, MI)) heom_
         }
         // ---- the next ADO's K neighbours: in flight through the exchange, the stores and its commutator ----
         if (AHEAD && more) {
-            if (mbar_wait(bars + ((it & 1) ^ 1), ((it + 1) >> 1) & 1)) load_k(slot_n, 0);
+            if (arrived(it + 1)) load_k(slot_n, 0);
             else failed = true;
         }
         // ---- the handed-over sector's terms to its owner ----
@@ -766,9 +777,13 @@ __global__ void __launch_bounds__(kRowWarps * 32, row_blocks(HK, SLT, MI)) heom_
             ci = ni;
         }
     }
-    // a warp whose wait expired flags the launch as failed and leaves; every copy it issued was either waited
-    // for or is the one whose wait has just run to its limit
-    if (failed && lane == 0) *static_cast<volatile int*>(dp.err) = 1;
+    // a warp whose wait expired flags the launch as failed; before it leaves, the copies that no wait has seen arrive
+    // (ADO it's, and the next one's where it was issued before that wait) get their time to land
+    if (failed) {
+        mbar_wait(bars + (it & 1), (it >> 1) & 1, 1 << 24);
+        if (!AHEAD && u + stride < nodes) mbar_wait(bars + ((it & 1) ^ 1), ((it + 1) >> 1) & 1, 1 << 24);
+        if (lane == 0) *static_cast<volatile int*>(dp.err) = 1;
+    }
 }
 
 // ---------------------------------------------------------------------------
