@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "heom_b200.h"
+#include "device_memory.hpp"
 #include "heom_kernels.cuh"
 #include "heom_lockstep.cuh"
 #include "host/heom_host.hpp"
@@ -28,6 +29,7 @@ namespace {
 }
 
 using heomk::PairParams;
+using heomrt::DevBuf;
 
 namespace {
 
@@ -65,32 +67,6 @@ constexpr double kProdBeta[4][2] = {
     {0.4573733434972976, -0.23510048799854266},
     {0.04262665650270243, -0.3946329531721134},
     {0.04262665650270243, 0.3946329531721134},
-};
-
-template <typename T>
-struct DevBuf {
-    T* p = nullptr;
-    size_t n = 0;
-    ~DevBuf() { reset(); }
-    void reset()
-    {
-        if (p) cudaFree(p);
-        p = nullptr;
-        n = 0;
-    }
-    int alloc(size_t count)
-    {
-        reset();
-        if (count == 0) count = 1;
-        cudaError_t e = cudaMalloc(&p, count * sizeof(T));
-        if (e != cudaSuccess) {
-            p = nullptr;
-            return fail(HEOM_E_NOMEM, "cudaMalloc of %zu bytes failed: %s", count * sizeof(T),
-                        cudaGetErrorString(e));
-        }
-        n = count;
-        return 0;
-    }
 };
 
 // Flags that kernels set and the host reads after the stream has drained: mapped pinned memory, so that a call that
@@ -2694,8 +2670,7 @@ struct heom_adjoint {
     int grid = 0, bpi = 0;     // blocks of the gradient kernel, per instance
     size_t grad_smem = 0;
     DevBuf<double2> cps, seg, scratch, ga, gb, toplog;
-    DevBuf<double2> ring;      // adjoint states of a group of steps (4 group of them; small hierarchies)
-    int64_t group = 0;         // steps whose gradient contributions are one launch (0: one launch per factor)
+    heomrt::AdjointRing<double2> ring; // adjoint states of a group of steps (four a step; small hierarchies)
     int64_t cap_cps = 0, cap_seg = 0, cap_rows = 0;
     int64_t mem_limit = 0;     // bytes for the sweep's states (0: free device memory)
     int64_t rec_slots = 0;     // recursive-checkpointing slots of the last sweep (0: sqrt layout)
@@ -2907,10 +2882,10 @@ int adj_seg_backward(heom_adjoint* A, double dt, int64_t len)
         return launch_stage(h, EPI_AXPY_SELF, in, nullptr, out, nullptr,
                             make_double2(dt * kProdBeta[k][0], -dt * kProdBeta[k][1]), 0, &A->tabs);
     };
-    if (A->group > 0) {
-        double2* ring = A->ring.p;
+    if (A->ring.group > 0) {
+        double2* ring = A->ring.states.p;
         for (int64_t j = len; j > 0;) { // steps j - 1, j - 2, ... of the segment
-            const int64_t steps = std::min<int64_t>(j, A->group), m = 4 * steps;
+            const int64_t steps = std::min<int64_t>(j, A->ring.group), m = 4 * steps;
             for (int64_t f = 0; f < m; ++f) {
                 const bool last = f + 1 == m;
                 if (last)
@@ -3174,14 +3149,16 @@ int heom_adjoint_gradient(heom_adjoint* A, const double* rho0, const double* obs
     // Small hierarchies: the gradient launches of a few steps are one, over a ring of adjoint states of at most
     // kRingBytes. A launch over 6435 ADOs leaves a warp three of them and is prologue, tail and latency (7 sites, depth
     // 8: 17 us a factor alone); from 16 MB a state a launch fills the device by itself. The ring takes no room from the
-    // checkpoints.
+    // checkpoints: an old one counts as memory to be had, and a new one fits in the slack.
     int64_t slots = 0, group = A->mem_limit == 0 ? std::min<int64_t>(S, (int64_t)(kRingBytes / (4 * st * 16))) : 0;
     // (free memory, whose query can take a millisecond, is of no interest while the last call's buffers do)
-    if (A->mem_limit != 0 || !A->ga.p || ncp > A->cap_cps || 4 * S > A->cap_seg || 4 * (size_t)group * st > A->ring.n) {
+    if (A->mem_limit != 0 || !A->ga.p || ncp > A->cap_cps || 4 * S > A->cap_seg ||
+        4 * (size_t)group * st > A->ring.states.n) {
         size_t free_b = 0, total_b = 0;
         CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
         const double sb = (double)st * 16.0;
-        const double held = (double)(A->cap_cps + A->cap_seg + (A->ga.p ? 3 : 0)) * sb;
+        const double held =
+            (double)(A->cap_cps + A->cap_seg + (A->ga.p ? 3 : 0)) * sb + (double)A->ring.states.n * 16.0;
         const double slack = std::max(512.0 * 1024 * 1024, 0.02 * (double)total_b);
         const double budget =
             A->mem_limit > 0 ? (double)A->mem_limit : std::max(0.0, (double)free_b - slack) + held;
@@ -3193,20 +3170,10 @@ int heom_adjoint_gradient(heom_adjoint* A, const double* rho0, const double* obs
             S = 1;
             ncp = slots;
         }
-        if (slots > 0 || (A->ring.n < 4 * (size_t)group * st &&
-                          (double)free_b < (double)(ncp + 4 * S + 3) * sb + 2.0 * kRingBytes))
-            group = 0;
+        if (slots > 0) group = 0;
     }
     A->rec_slots = slots;
-    if (group != A->group) {
-        A->drop_graphs();
-        A->group = group;
-        if (4 * (size_t)group * st > A->ring.n || group == 0) {
-            A->ring.reset();
-            if (group > 0)
-                if (int rc = A->ring.alloc(4 * (size_t)group * st)) return rc;
-        }
-    }
+    if (A->ring.resize(group, 4 * st)) A->drop_graphs();
     // the gradients to accumulate (NULL outputs are skipped); the captured graphs hold them
     const int want_h = grad_h ? 1 : 0, want_bath = (grad_lambda || grad_gamma) ? 1 : 0;
     if (want_h != A->want_h || want_bath != A->want_bath) {
@@ -3310,7 +3277,7 @@ int heom_adjoint_gradient(heom_adjoint* A, const double* rho0, const double* obs
     }
 
     // ---- backward (sqrt layout; the recursive sweep has run above) ----
-    double2* gcur = A->group > 0 ? A->ring.p : A->ga.p; // adj_seg_backward's state between segments
+    double2* gcur = A->ring.group > 0 ? A->ring.states.p : A->ga.p; // adj_seg_backward's state between segments
     if (slots == 0) {
         CUDA_TRY(cudaMemsetAsync(A->partial.p, 0, (size_t)A->grid * (NN + 2) * 16, h->stream));
         CUDA_TRY(cudaMemsetAsync(gcur, 0, st * 16, h->stream));
