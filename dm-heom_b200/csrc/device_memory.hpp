@@ -4,6 +4,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <string>
+#include <utility>
 #include <cuda_runtime.h>
 #include "heom_b200.h"
 
@@ -33,6 +34,7 @@ struct DevBuf {
         if (count == 0) count = 1;
         cudaError_t e = cudaMalloc(&p, count * sizeof(T));
         if (e != cudaSuccess) {
+            cudaGetLastError(); // reported here: not for the next launch's check to find
             p = nullptr;
             char buf[160];
             snprintf(buf, sizeof buf, "cudaMalloc of %zu bytes failed: %s", count * sizeof(T), cudaGetErrorString(e));
@@ -41,8 +43,14 @@ struct DevBuf {
         n = count;
         return 0;
     }
-    // at least `count` elements; what is large enough is kept, contents and all
+    // at least `count` elements; what is large enough is kept, contents and all.  After a failure the buffer is empty
+    // and says so, and the next call tries again.
     int ensure(size_t count) { return p && n >= count ? 0 : alloc(count); }
+    void swap(DevBuf& o)
+    {
+        std::swap(p, o.p);
+        std::swap(n, o.n);
+    }
 };
 
 // The adjoint states of a group of steps, whose gradient contributions are then one launch.  The sweep works without
@@ -59,10 +67,7 @@ struct AdjointRing {
         const T* const at = states.p;
         if (want == 0) states.reset();
         group = want;
-        if (want > 0 && states.ensure((size_t)want * step) != 0) {
-            cudaGetLastError(); // dealt with: not for the next launch's check to find
-            group = 0;
-        }
+        if (want > 0 && states.ensure((size_t)want * step) != 0) group = 0;
         return group != had || states.p != at;
     }
 };

@@ -1096,7 +1096,7 @@ int build_pair_tables(heom_handle* h, bool lockstep = false)
             lt.ord[k] = (signed char)(d ? diag[nd++] : off[no++]);
         }
     }
-    if (int rc = h->d_pair.alloc(2 * P)) return rc;
+    if (int rc = h->d_pair.ensure(2 * P)) return rc;
     CUDA_TRY(cudaMemcpy(h->d_pair.p, h->pair_tab.data(), 2 * P * sizeof(int16_t), cudaMemcpyHostToDevice));
     return 0;
 }
@@ -1218,25 +1218,20 @@ int make_lockstep(heom_handle* h)
     // the instance-minor state first: if it cannot be had, the handle stays the batch handle it was
     const int64_t kp = (h->n_inst + 31) / 32 * 32;
     const size_t elems = (size_t)n0 * kp * 2 * h->P;
-    double2* ny = nullptr;
-    if (cudaMalloc(&ny, elems * sizeof(double2)) != cudaSuccess)
-        return fail(HEOM_E_NOMEM, "lockstep layout: cudaMalloc of %zu bytes failed", elems * sizeof(double2));
+    DevBuf<double2> ny;
+    if (int rc = ny.alloc(elems)) return rc;
     const std::vector<int64_t> tops(h->n_inst, h->top_int[0] - h->inst_base[0]);
     if (int rc = build_pair_tables(h, true)) {
         build_pair_tables(h);
-        cudaFree(ny);
         return rc;
     }
-    if (cudaMemset(ny, 0, elems * sizeof(double2)) != cudaSuccess ||
+    if (cudaMemset(ny.p, 0, elems * sizeof(double2)) != cudaSuccess ||
         cudaMemcpy(h->d_top.p, tops.data(), tops.size() * 8, cudaMemcpyHostToDevice) != cudaSuccess) {
         const cudaError_t err = cudaGetLastError();
         build_pair_tables(h);
-        cudaFree(ny);
         return fail(HEOM_E_CUDA, "lockstep layout: %s", cudaGetErrorString(err));
     }
-    h->y.data.reset();
-    h->y.data.p = ny;
-    h->y.data.n = elems;
+    h->y.data.swap(ny);
     h->inst_nodes = n0;
     h->kp = kp;
     for (auto& w : h->work) w.reset();
@@ -1584,13 +1579,11 @@ int heom_set_field(heom_handle* h, const double* dipole_plus, const double* dipo
     for (int q = 0; q < 2; ++q)
         h->pulses[q] = heomk::Pulse{pl[q]->efield, pl[q]->time_center, pl[q]->time_width, pl[q]->frequency,
                                     pl[q]->phase};
-    if (!h->d_dplus.p) {
-        if (int rc = h->d_dplus.alloc(N * N)) return rc;
-        if (int rc = h->d_dminus.alloc(N * N)) return rc;
-        if (int rc = h->field_hs.alloc((size_t)3 * K * N * N)) return rc;
-        if (int rc = h->field_frag.alloc((size_t)3 * K * heomk::frag_doubles(N))) return rc;
-        if (int rc = h->d_time.alloc(1)) return rc;
-    }
+    if (int rc = h->d_dplus.ensure(N * N)) return rc;
+    if (int rc = h->d_dminus.ensure(N * N)) return rc;
+    if (int rc = h->field_hs.ensure((size_t)3 * K * N * N)) return rc;
+    if (int rc = h->field_frag.ensure((size_t)3 * K * heomk::frag_doubles(N))) return rc;
+    if (int rc = h->d_time.ensure(1)) return rc;
     CUDA_TRY(cudaMemcpy(h->d_dplus.p, dp.data(), N * N * 16, cudaMemcpyHostToDevice));
     CUDA_TRY(cudaMemcpy(h->d_dminus.p, dm.data(), N * N * 16, cudaMemcpyHostToDevice));
     CUDA_TRY(cudaMemcpy(h->d_time.p, &h->time, 8, cudaMemcpyHostToDevice));
@@ -1820,13 +1813,15 @@ int heom_set_flow_buffers(heom_handle* h, heom_buffer* flow_from_above, heom_buf
     if (flow_from_above && flow_from_above == flow_from_below)
         return fail(HEOM_E_ARG, "the two flow buffers must differ");
     CUDA_TRY(cudaSetDevice(h->device));
-    if ((flow_from_above || flow_from_below) && !h->d_zero.p) {
+    if (flow_from_above || flow_from_below) {
         const size_t K = h->n_inst, N = h->N;
         size_t len = std::max<size_t>({K * heomk::frag_doubles((int)N), K * N * (N + 1), 2 * K * N * N, (size_t)6 * h->W * h->LS,
                                        (size_t)6 * h->W, (size_t)2 * h->nodes});
-        if (int rc = h->d_zero.alloc(len)) return rc;
-        CUDA_TRY(cudaMemset(h->d_zero.p, 0, len * 8));
-        if (int rc = h->flow_scratch.alloc(h->state_elems())) return rc;
+        if (h->d_zero.n < len) {
+            if (int rc = h->d_zero.alloc(len)) return rc;
+            CUDA_TRY(cudaMemset(h->d_zero.p, 0, len * 8));
+        }
+        if (int rc = h->flow_scratch.ensure(h->state_elems())) return rc;
     }
     h->flow_above = flow_from_above;
     h->flow_below = flow_from_below;
@@ -1962,8 +1957,7 @@ int heom_propagate(heom_handle* h, double dt, int64_t steps, int64_t observe_eve
     CUDA_TRY(cudaSetDevice(h->device));
     const int64_t rows = steps / observe_every + 1;
     const int64_t nn = (int64_t)h->N * h->N * h->n_inst;
-    if ((int64_t)h->toplog.n < rows * nn)
-        if (int rc = h->toplog.alloc(rows * nn)) return rc;
+    if (int rc = h->toplog.ensure(rows * nn)) return rc;
     heomk::heom_record_top<<<h->n_inst, 128, 0, h->stream>>>(h->toplog.p, h->y.data.p, h->d_pair.p, h->d_top.p, h->N,
                                                              h->P, 0, h->kp, 0);
     h->launches++;
@@ -2575,8 +2569,7 @@ int heom_ensemble_propagate(heom_ensemble* e, double dt, int64_t steps, int64_t 
     const int64_t rows = steps / observe_every + 1;
     for (heom_handle* h : e->cls) {
         const int64_t nn = (int64_t)h->N * h->N * h->n_inst;
-        if ((int64_t)h->toplog.n < rows * nn)
-            if (int rc = h->toplog.alloc(rows * nn)) return rc;
+        if (int rc = h->toplog.ensure(rows * nn)) return rc;
         CUDA_TRY(cudaStreamSynchronize(h->stream));
     }
     auto record = [&](int64_t row) -> int {
@@ -2671,13 +2664,11 @@ struct heom_adjoint {
     size_t grad_smem = 0;
     DevBuf<double2> cps, seg, scratch, ga, gb, toplog;
     heomrt::AdjointRing<double2> ring; // adjoint states of a group of steps (four a step; small hierarchies)
-    int64_t cap_cps = 0, cap_seg = 0, cap_rows = 0;
     int64_t mem_limit = 0;     // bytes for the sweep's states (0: free device memory)
     int64_t rec_slots = 0;     // recursive-checkpointing slots of the last sweep (0: sqrt layout)
     int want_h = 1, want_bath = 1; // gradients the sweep accumulates (from the output pointers)
     DevBuf<double> d_w;        // loss weights [steps + 1]
     DevBuf<int64_t> d_base;    // step offset of the segment being run (read by the captured kernels)
-    int64_t cap_w = 0;
     // captured graphs per segment length: [0] forward with tops, [1] stage-input recompute, [2] backward
     struct Graphs {
         int64_t len = 0;
@@ -3152,13 +3143,13 @@ int heom_adjoint_gradient(heom_adjoint* A, const double* rho0, const double* obs
     // checkpoints: an old one counts as memory to be had, and a new one fits in the slack.
     int64_t slots = 0, group = A->mem_limit == 0 ? std::min<int64_t>(S, (int64_t)(kRingBytes / (4 * st * 16))) : 0;
     // (free memory, whose query can take a millisecond, is of no interest while the last call's buffers do)
-    if (A->mem_limit != 0 || !A->ga.p || ncp > A->cap_cps || 4 * S > A->cap_seg ||
-        4 * (size_t)group * st > A->ring.states.n) {
+    if (A->mem_limit != 0 || A->scratch.n < st || A->cps.n < ncp * st || A->seg.n < 4 * S * st ||
+        A->ring.states.n < 4 * (size_t)group * st) {
         size_t free_b = 0, total_b = 0;
         CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
         const double sb = (double)st * 16.0;
         const double held =
-            (double)(A->cap_cps + A->cap_seg + (A->ga.p ? 3 : 0)) * sb + (double)A->ring.states.n * 16.0;
+            16.0 * (double)(A->cps.n + A->seg.n + A->ga.n + A->gb.n + A->scratch.n + A->ring.states.n);
         const double slack = std::max(512.0 * 1024 * 1024, 0.02 * (double)total_b);
         const double budget =
             A->mem_limit > 0 ? (double)A->mem_limit : std::max(0.0, (double)free_b - slack) + held;
@@ -3182,37 +3173,23 @@ int heom_adjoint_gradient(heom_adjoint* A, const double* rho0, const double* obs
         A->want_bath = want_bath;
     }
     // the captured graphs hold buffer addresses: any reallocation drops them
-    const bool shrink = slots > 0 && (A->cap_cps > ncp || A->cap_seg > 4);
-    if (shrink || ncp > A->cap_cps || 4 * S > A->cap_seg || steps + 1 > A->cap_rows || steps + 1 > A->cap_w)
+    const bool shrink = slots > 0 && (A->cps.n > ncp * st || A->seg.n > 4 * st);
+    const size_t rows = (size_t)(steps + 1) * NN * K;
+    if (shrink || A->cps.n < ncp * st || A->seg.n < 4 * S * st || A->toplog.n < rows || (int64_t)A->d_w.n < steps + 1 ||
+        A->ga.n < st || A->gb.n < st || A->scratch.n < st || !A->d_base.p)
         A->drop_graphs();
     if (shrink) { // release the sqrt layout before the recursive one takes its place
         A->cps.reset();
         A->seg.reset();
-        A->cap_cps = A->cap_seg = 0;
     }
-    if (ncp > A->cap_cps) {
-        if (int rc = A->cps.alloc(ncp * st)) return rc;
-        A->cap_cps = ncp;
-    }
-    if (4 * S > A->cap_seg) {
-        if (int rc = A->seg.alloc(4 * S * st)) return rc;
-        A->cap_seg = 4 * S;
-    }
-    if (!A->ga.p) {
-        if (int rc = A->ga.alloc(st)) return rc;
-        if (int rc = A->gb.alloc(st)) return rc;
-        if (int rc = A->scratch.alloc(st)) return rc;
-    }
-    if (steps + 1 > A->cap_rows) {
-        if (int rc = A->toplog.alloc((steps + 1) * NN * K)) return rc;
-        A->cap_rows = steps + 1;
-    }
-    if (steps + 1 > A->cap_w) {
-        if (int rc = A->d_w.alloc(steps + 1)) return rc;
-        A->cap_w = steps + 1;
-    }
-    if (!A->d_base.p)
-        if (int rc = A->d_base.alloc(1)) return rc;
+    if (int rc = A->cps.ensure(ncp * st)) return rc;
+    if (int rc = A->seg.ensure(4 * S * st)) return rc;
+    if (int rc = A->ga.ensure(st)) return rc;
+    if (int rc = A->gb.ensure(st)) return rc;
+    if (int rc = A->scratch.ensure(st)) return rc;
+    if (int rc = A->toplog.ensure(rows)) return rc;
+    if (int rc = A->d_w.ensure(steps + 1)) return rc;
+    if (int rc = A->d_base.ensure(1)) return rc;
     if (int rc = prepare_scheme(h)) return rc;
     {
         // resolve both stage kernels' launch shapes outside of any capture

@@ -72,8 +72,27 @@ static void ring()
     CHECK(r.resize(4, 40) && r.group == 4 && r.states.p);
 }
 
+static void buffers()
+{
+    heomrt::DevBuf<double> a, b;
+    CHECK(a.ensure(100) == 0 && a.n == 100);
+    const double* at = a.p;
+    CHECK(a.ensure(60) == 0 && a.p == at && a.n == 100); // kept: what holds its address stays valid
+    // no memory for a larger one: the buffer is empty and says so, and no error waits for the next launch's check
+    no_memory(1);
+    CHECK(a.ensure(200) == HEOM_E_NOMEM && !a.p && a.n == 0);
+    CHECK(cudaGetLastError() == cudaSuccess);
+    // the size it had before the failure is not there any more, and is asked for again
+    const long before = mallocs;
+    CHECK(a.ensure(60) == 0 && a.p && a.n == 60 && mallocs == before + 1);
+    CHECK(b.ensure(5) == 0);
+    a.swap(b);
+    CHECK(a.n == 5 && b.n == 60 && a.p != b.p);
+}
+
 int main()
 {
+    buffers();
     ring();
     CHECK(live.empty());
     printf("%s\n", bad ? "FAILED" : "ok");
