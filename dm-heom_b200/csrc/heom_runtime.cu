@@ -21,6 +21,7 @@
 #include "device_memory.hpp"
 #include "heom_kernels.cuh"
 #include "heom_lockstep.cuh"
+#include "host_flag.hpp"
 #include "host/heom_host.hpp"
 
 namespace {
@@ -30,6 +31,7 @@ namespace {
 
 using heomk::PairParams;
 using heomrt::DevBuf;
+using heomrt::HostFlag;
 
 namespace {
 
@@ -67,67 +69,6 @@ constexpr double kProdBeta[4][2] = {
     {0.4573733434972976, -0.23510048799854266},
     {0.04262665650270243, -0.3946329531721134},
     {0.04262665650270243, 0.3946329531721134},
-};
-
-// Flags that kernels set and the host reads after the stream has drained: mapped pinned memory, so that a call that
-// checks one needs no copy of its own.  Page-locking takes longer than the rest of a small handle's creation, so the
-// handles share a page of flags, which goes with the last of them.
-struct FlagPage {
-    static constexpr int kFlags = 1024;
-    int* host = nullptr;
-    std::vector<int> unused;
-    std::mutex mu;
-    ~FlagPage()
-    {
-        if (host) cudaFreeHost(host);
-    }
-};
-std::mutex g_flag_mu;
-std::weak_ptr<FlagPage> g_flag_page; // the page that new flags come from
-
-struct HostFlag {
-    std::shared_ptr<FlagPage> page;
-    int index = -1;
-    int* dev = nullptr;
-    ~HostFlag()
-    {
-        if (!page) return;
-        std::lock_guard<std::mutex> lock(page->mu);
-        page->unused.push_back(index);
-    }
-    int alloc()
-    {
-        std::lock_guard<std::mutex> lock(g_flag_mu);
-        std::shared_ptr<FlagPage> pg = g_flag_page.lock();
-        bool full = !pg;
-        if (pg) {
-            std::lock_guard<std::mutex> pl(pg->mu);
-            full = pg->unused.empty();
-        }
-        if (full) {
-            pg = std::make_shared<FlagPage>();
-            const cudaError_t e =
-                cudaHostAlloc(&pg->host, FlagPage::kFlags * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable);
-            if (e != cudaSuccess) {
-                pg->host = nullptr;
-                return fail(HEOM_E_NOMEM, "mapped flags: %s", cudaGetErrorString(e));
-            }
-            for (int q = FlagPage::kFlags - 1; q >= 0; --q) pg->unused.push_back(q);
-            g_flag_page = pg;
-        }
-        int* base = nullptr; // this device's address of the page
-        const cudaError_t e = cudaHostGetDevicePointer(&base, pg->host, 0);
-        if (e != cudaSuccess) return fail(HEOM_E_CUDA, "mapped flags: %s", cudaGetErrorString(e));
-        std::lock_guard<std::mutex> pl(pg->mu);
-        index = pg->unused.back();
-        pg->unused.pop_back();
-        page = pg;
-        dev = base + index;
-        clear();
-        return 0;
-    }
-    void clear() { static_cast<volatile int*>(page->host)[index] = 0; }
-    bool set() const { return static_cast<volatile int*>(page->host)[index] != 0; }
 };
 
 typedef void (*dmma_fn_t)(const heomk::DmmaParams);
@@ -1481,8 +1422,8 @@ int heom_create_batch(const heom_instance_desc* descs, int32_t count, const heom
     h->xfer_ados = std::max<int64_t>(1, std::min<int64_t>(h->nodes, (int64_t(64) << 20) / (nn * 16)));
     if (int rc = h->xfer.alloc((size_t)h->xfer_ados * nn)) return rc;
     if (int rc = h->topbuf.alloc((size_t)count * nn)) return rc;
-    if (int rc = h->flag.alloc()) return rc;
-    if (int rc = h->err.alloc()) return rc;
+    if (int rc = h->flag.alloc(h->device)) return rc;
+    if (int rc = h->err.alloc(h->device)) return rc;
     *out = h.release();
     return 0;
 }
