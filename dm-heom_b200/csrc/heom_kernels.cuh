@@ -1272,9 +1272,14 @@ __global__ void heom_write_top(double2* __restrict__ y, const double2* __restric
 //           their derivatives (dpss, dgamma0, dchat, dkhat).
 // One warp per ADO; its lanes take the (state, column pair) threads of the
 // stage kernels in turn, so that the look-ups of a slot serve four elements, and
-// the derivative tables lie in shared memory.  Latency bounds it: 4 instances of
-// 9 states, 715 ADOs each, 18 us a factor with a lane per sector and its tables
-// in global memory.  The blocks are split
+// the derivative tables lie in shared memory.  Latency bounds it, so that two
+// blocks on an SM count for more than the 32 bytes that 128 registers spill, and
+// a warp's sums lie where its tiles were (16 states: 90 KB a block).  Whole
+// gradient calls, one B200, with one block of 158 registers -> with two: 4
+// instances of 9 states, 715 ADOs each, 40 steps 7220 -> 6910 us; 12 states, two
+// slots, 20,475 ADOs, 8 steps 10,840 -> 9150; 16 states, 4845 ADOs, 20 steps
+// 10,900 -> 9540 (a lane per sector, tables in global memory, two blocks of 126
+// registers: 8410, 12,200 and 9990).  The blocks are split
 // among the instances of the handle (each block sweeps one instance's ADOs),
 // and every block adds weight * (its sum) to its own row of `partial`
 // (deterministic; summed per instance on the host at the end).
@@ -1309,22 +1314,22 @@ struct GradParams {
 struct GradLane {
     short r, diag, pso, psg, e1, e2, q1, q2, gr, gc, twin, pad; // diag 1: the owned sector is diagonal, 2: the other
 };
-__host__ __device__ inline int grad_warp_bytes(int n) { return 2 * n * (n + 1) * 16; }
+// a warp's two tiles [n][n+1]; at the end of a factor its n*n + 2 sums lie there
+__host__ __device__ constexpr int grad_warp_bytes(int n) { return 2 * n * (n + 1) * 16; }
 __host__ inline size_t grad_smem_bytes(int n, int W, int LS)
 {
-    return (size_t)kCtaWarps * grad_warp_bytes(n) + (size_t)(kCtaWarps + 1) * (n * n + 2) * 16 +
+    return (size_t)kCtaWarps * grad_warp_bytes(n) + (size_t)(n * n + 2) * 16 +
            (size_t)(2 * n * n + 5 * W) * 16 + (size_t)((LS + 2) & ~1) * 8 + (size_t)n * ((n + 1) / 2) * sizeof(GradLane);
 }
 
-__global__ void __launch_bounds__(kCtaWarps * 32) heom_adjoint_grad(const __grid_constant__ GradParams g)
+__global__ void __launch_bounds__(kCtaWarps * 32, 2) heom_adjoint_grad(const __grid_constant__ GradParams g)
 {
     extern __shared__ __align__(128) unsigned char smem[];
     const int N = g.N, P = g.P, W = g.W, SL = g.SL, NN = N * N, LD = N + 1;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     double2* At = reinterpret_cast<double2*>(smem + warp * grad_warp_bytes(N)); // [N][N+1]
     double2* Wt = At + N * LD;
-    double2* red = reinterpret_cast<double2*>(smem + kCtaWarps * grad_warp_bytes(N)); // [warps][NN+2]
-    double2* acc = red + kCtaWarps * (NN + 2);                                         // [NN+2]
+    double2* acc = reinterpret_cast<double2*>(smem + kCtaWarps * grad_warp_bytes(N)); // [NN+2]
     // derivative tables, lambda and gamma side by side: dg0 [NN][2], dkhat side i and side j [W][4], dchat [W]
     double2* s_dg = acc + NN + 2;
     double2* s_dk = s_dg + 2 * NN;
@@ -1500,7 +1505,7 @@ __global__ void __launch_bounds__(kCtaWarps * 32) heom_adjoint_grad(const __grid
             __syncwarp();
         }
         // block sum in a fixed order, then weight * sum into this block's row
-        double2* mine = red + warp * (NN + 2);
+        double2* mine = At; // [NN+2], where the warp's tiles were
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
             if (b >= nblk) continue;
@@ -1526,8 +1531,9 @@ __global__ void __launch_bounds__(kCtaWarps * 32) heom_adjoint_grad(const __grid
         for (int q = threadIdx.x; q < NN + 2; q += blockDim.x) {
             double2 s = z0;
             for (int v = 0; v < kCtaWarps; ++v) {
-                s.x += red[v * (NN + 2) + q].x;
-                s.y += red[v * (NN + 2) + q].y;
+                const double2 m = reinterpret_cast<const double2*>(smem + v * grad_warp_bytes(N))[q];
+                s.x += m.x;
+                s.y += m.y;
             }
             acc[q].x += wgt.x * s.x - wgt.y * s.y;
             acc[q].y += wgt.x * s.y + wgt.y * s.x;
@@ -1558,8 +1564,7 @@ __global__ void __launch_bounds__(kCtaWarps * 32, 2) heom_row_grad(const __grid_
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     double2* At = reinterpret_cast<double2*>(smem + warp * grad_warp_bytes(N)); // [N][N+1]
     double2* Wt = At + N * LD;
-    double2* red = reinterpret_cast<double2*>(smem + kCtaWarps * grad_warp_bytes(N)); // [warps][NN+2]
-    double2* acc = red + kCtaWarps * (NN + 2);                                         // [NN+2]
+    double2* acc = reinterpret_cast<double2*>(smem + kCtaWarps * grad_warp_bytes(N)); // [NN+2]
 
     // ---- this lane's place (heom_dmma_stage) ----
     const int r = lane >> 2, t = lane & 3;
@@ -1723,7 +1728,7 @@ __global__ void __launch_bounds__(kCtaWarps * 32, 2) heom_row_grad(const __grid_
             __syncwarp();
         }
         // the coefficients' derivatives, then the block's sum in a fixed order, times the factor's weight
-        double2* mine = red + warp * (NN + 2);
+        double2* mine = At; // [NN+2], where the warp's tiles were
         if (r < N && 2 * t < N) mine[r * N + 2 * t] = make_double2(zr0, zi0);
         if (r < N && 2 * t + 1 < N) mine[r * N + 2 * t + 1] = make_double2(zr1, zi1);
         double2 d[2] = {z0, sd}; // lambda, gamma
@@ -1754,8 +1759,9 @@ __global__ void __launch_bounds__(kCtaWarps * 32, 2) heom_row_grad(const __grid_
         for (int q = threadIdx.x; q < NN + 2; q += blockDim.x) {
             double2 s = z0;
             for (int v = 0; v < kCtaWarps; ++v) {
-                s.x += red[v * (NN + 2) + q].x;
-                s.y += red[v * (NN + 2) + q].y;
+                const double2 m = reinterpret_cast<const double2*>(smem + v * grad_warp_bytes(N))[q];
+                s.x += m.x;
+                s.y += m.y;
             }
             acc[q].x += wgt.x * s.x - wgt.y * s.y;
             acc[q].y += wgt.x * s.y + wgt.y * s.x;

@@ -3033,7 +3033,7 @@ int heom_adjoint_create_batch(const heom_system_desc* systems, int32_t count, co
     CUDA_TRY(cudaSetDevice(h->device));
     if (int rc = adj_tables(A.get(), sp[0])) return rc;
     if (int rc = A->obs.alloc((size_t)count * h->N * h->N)) return rc;
-    // gradient kernel: every instance gets the same number of blocks, about two waves in all
+    // gradient kernel: every instance gets the same number of blocks, about two on each SM in all (one wave)
     int64_t max_nodes = 1;
     for (int k = 0; k < count; ++k) max_nodes = std::max(max_nodes, h->inst_base[k + 1] - h->inst_base[k]);
     A->bpi = (int)std::max<int64_t>(1, std::min<int64_t>((max_nodes + heomk::kCtaWarps - 1) / heomk::kCtaWarps,

@@ -39,6 +39,10 @@ int main()
                 if (NW % 4 || NW < 2 * W || TWB % 16 || TWB < W) { printf("bad pads W=%d\n", W); ++bad; }
                 ++checked;
             }
+        // gradient kernels: a warp's sums fit where its tiles were, and two blocks an SM (228 KB, 1 KB of them the
+        // system's for each block) at the widest tables that a handle takes
+        if ((n * n + 2) * 16 > heomk::grad_warp_bytes(n)) { printf("bad gradient sums n=%d\n", n); ++bad; }
+        if (2 * (heomk::grad_smem_bytes(n, 255, 251) + 1024) > 228 * 1024) { printf("bad gradient blocks n=%d\n", n); ++bad; }
         // tile positions: inside the row, one per element
         {
             int used[16 * 20] = {0};
