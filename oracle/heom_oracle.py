@@ -18,7 +18,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
-from dataclasses import dataclass, field
+from dataclasses import dataclass, field, replace
 
 import numpy as np
 
@@ -380,6 +380,20 @@ def ref_derivative(prob: Problem, y: np.ndarray, threads=None, mode=0, out_coeff
     if rc != 0:
         raise RuntimeError("refcl_heom_ode failed")
     return out, accb
+
+
+def neighbour_terms(prob: Problem, y: np.ndarray, threads=None):
+    """(full, plus, minus): the derivative and its plus and minus terms (heom_ode.cl:183-259, :280-403), from the
+    reference's kernel built with HEOM_ODE_DISABLE_PLUS / _MINUS where that is there, else from the oracle: without
+    plus terms when no ADO has a plus neighbour, without minus terms too when all tuple entries are 0."""
+    if ref_lib() is not None:
+        full, _ = ref_derivative(prob, y, threads)
+        return full, full - ref_derivative(prob, y, threads, mode=3)[0], full - ref_derivative(prob, y, threads, mode=4)[0]
+    g = replace(prob.graph, first_non_plus=0)
+    no_plus = replace(prob, graph=g)
+    neither = replace(prob, graph=replace(g, tuples=np.zeros_like(g.tuples)))
+    full, rest = derivative(prob, y, threads), derivative(no_plus, y, threads)
+    return full, full - rest, rest - derivative(neither, y, threads)
 
 
 def ref_weighted_add(prob: Problem, h, y, coeffs, ks, threads=None, fast=False):

@@ -176,9 +176,10 @@ def test_app_tracks_flows_like_the_reference_solver(tmp_path):
     stepping zeroes them at every step and accumulates dt b_i x the plus and
     minus terms of every evaluation; the flow file holds, at every
     observation, the sum over ADOs of each buffer's hierarchy norm after the
-    last step.  Checked against the reference's own kernel terms (the kernel
-    built with HEOM_ODE_DISABLE_PLUS / _MINUS) over the classical RK4 stage
-    inputs of the oracle; the populations are those of the untracked run."""
+    last step.  Checked against the terms of the reference's own kernel (built
+    with HEOM_ODE_DISABLE_PLUS / _MINUS), or the oracle's where that is not
+    built, over the classical RK4 stage inputs; the populations are those of
+    the untracked run."""
     cfg = FMO_CFG.replace("track_flows=false", "track_flows=true").replace("flow_filename=", "flow_filename=f.dat")
     (tmp_path / "heom.cfg").write_text(cfg)
     (tmp_path / "rt.cfg").write_text("[cuda]\ndevice_index=0\n")
@@ -194,24 +195,16 @@ def test_app_tracks_flows_like_the_reference_solver(tmp_path):
     assert hf == ["time", "flow_from_above_norm", "flow_from_below_norm"]
     assert f.shape == (4, 3)  # one row per observation after t = 0
 
-    def terms(v):
-        full, _ = ho.ref_derivative(prob, v)
-        return full - ho.ref_derivative(prob, v, mode=3)[0], full - ho.ref_derivative(prob, v, mode=4)[0]
-
     y = prob.initial_state()
     for obs_row in range(4):
         for step in range(5):
-            k1, _ = ho.ref_derivative(prob, y)
-            s2 = y + 0.5 * dt * k1
-            k2, _ = ho.ref_derivative(prob, s2)
-            s3 = y + 0.5 * dt * k2
-            k3, _ = ho.ref_derivative(prob, s3)
-            s4 = y + dt * k3
-            k4, _ = ho.ref_derivative(prob, s4)
+            k1, p1, m1 = ho.neighbour_terms(prob, y)
+            k2, p2, m2 = ho.neighbour_terms(prob, y + 0.5 * dt * k1)
+            k3, p3, m3 = ho.neighbour_terms(prob, y + 0.5 * dt * k2)
+            k4, p4, m4 = ho.neighbour_terms(prob, y + dt * k3)
             above = np.zeros_like(y)
             below = np.zeros_like(y)
-            for s, b in zip((y, s2, s3, s4), (1 / 6, 1 / 3, 1 / 3, 1 / 6)):
-                p, m = terms(s)
+            for p, m, b in ((p1, m1, 1 / 6), (p2, m2, 1 / 3), (p3, m3, 1 / 3), (p4, m4, 1 / 6)):
                 above += dt * b * p
                 below += dt * b * m
             y = y + dt / 6 * (k1 + 2 * k2 + 2 * k3 + k4)
