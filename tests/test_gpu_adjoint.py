@@ -419,3 +419,143 @@ def test_adjoint_at_full_size_matches_oracle_tangents():
     pg, mg = problem(h, lam, 1.0 / (g + dg), 1, depth), problem(h, lam, 1.0 / (g - dg), 1, depth)
     ref_g = tangent(lambda v: (L(pg, v) - L(mg, v)) / (2 * dg))
     assert abs(gpu["gamma"] - ref_g) <= 1e-6 * abs(ref_g), (gpu["gamma"], ref_g)
+
+
+def tangent_gradients(n, h, lam, inv, m, depth, dt_fs, steps, rho0, obs, w, omega, coupling, entries, tops):
+    """J and its gradients by forward-mode tangents of the oracle's RK4 steps, with no matrix of the operator: along
+    H entries (L is affine in H: L' v = i/hbar (v E - E v) on every ADO), elements of rho0 (the loss is linear in the
+    state), and lambda and gamma (central differences of oracle operators, 1e-4 relative)."""
+    hbar = 1.05457148e-34  # the reference's value (common.cl, constants.hpp)
+    dt = dt_fs * 1e-15
+
+    def prob(lam_=lam, inv_=inv):
+        return ho.build_problem(ho.make_system(h, [lam_] * n, [inv_] * n, [omega] * n, m, 300.0, depth,
+                                               coupling=coupling))
+
+    base = prob()
+    L = lambda p, v: ho.derivative(p, v, threads=1)
+    loss = lambda v: float(np.real(np.vdot(obs.reshape(-1), v.view(np.complex128)[: n * n])))
+
+    def start(top):
+        y = np.zeros(base.state_len)
+        y.view(np.complex128)[: n * n] = top.reshape(-1)
+        return y
+
+    def sweep(y):  # J and the stage inputs of every step
+        J, stages = w[0] * loss(y), []
+        for k in range(steps):
+            k1 = L(base, y)
+            s2 = y + 0.5 * dt * k1
+            k2 = L(base, s2)
+            s3 = y + 0.5 * dt * k2
+            k3 = L(base, s3)
+            s4 = y + dt * k3
+            stages.append((y, s2, s3, s4))
+            y = y + dt / 6.0 * (k1 + 2.0 * k2 + 2.0 * k3 + L(base, s4))
+            J += w[k + 1] * loss(y)
+        return J, stages
+
+    J, stages = sweep(start(rho0))
+
+    def tangent(dL):
+        dy, dJ = np.zeros(base.state_len), 0.0
+        for k in range(steps):
+            y0, s2, s3, s4 = stages[k]
+            dk1 = L(base, dy) + dL(y0)
+            dk2 = L(base, dy + 0.5 * dt * dk1) + dL(s2)
+            dk3 = L(base, dy + 0.5 * dt * dk2) + dL(s3)
+            dk4 = L(base, dy + dt * dk3) + dL(s4)
+            dy = dy + dt / 6.0 * (dk1 + 2.0 * dk2 + 2.0 * dk3 + dk4)
+            dJ += w[k + 1] * loss(dy)
+        return dJ
+
+    def along(a, b, part):
+        E = np.zeros((n, n), complex)
+        E[a, b] = part * INVCM
+
+        def apply(v):
+            s = v.view(np.complex128).reshape(-1, n, n)
+            return np.ascontiguousarray(1j / hbar * (s @ E - E @ s)).reshape(-1).view(np.float64)
+        return apply
+
+    gh = {(a, b): tangent(along(a, b, 1.0)) + 1j * tangent(along(a, b, 1j)) for a, b in entries}
+    dl, g = 1e-4 * lam, 1.0 / inv
+    dg = 1e-4 * g
+    pl, ml, pg, mg = prob(lam + dl), prob(lam - dl), prob(inv_=1.0 / (g + dg)), prob(inv_=1.0 / (g - dg))
+    gl = tangent(lambda v: (L(pl, v) - L(ml, v)) / (2 * dl))
+    gg = tangent(lambda v: (L(pg, v) - L(mg, v)) / (2 * dg))
+    gr = {}
+    for a, b in tops:
+        e = np.zeros((n, n), complex)
+        e[a, b] = 1.0
+        gr[(a, b)] = sweep(start(e))[0] + 1j * sweep(start(1j * e))[0]
+    return J, gh, gl, gg, gr
+
+
+@pytest.mark.parametrize("n,m,depth,bps,cplx", [
+    # up to 8 states, one or two slots per state (a bath on two states has its slot in both)
+    (1, 1, 3, 1, False), (2, 1, 3, 1, False), (2, 2, 3, 1, True), (5, 1, 2, 2, False), (6, 1, 2, 1, False),
+    (6, 2, 2, 1, False), (7, 2, 2, 1, True), (8, 1, 2, 1, False), (8, 2, 2, 1, True),
+    # up to 8 states, three slots and more
+    (1, 3, 3, 1, False), (2, 4, 2, 1, False), (3, 2, 2, 2, True), (4, 3, 2, 1, False), (8, 3, 1, 1, False),
+    # more than 8 states: odd and even, one slot and more, a bath on two states
+    (9, 2, 2, 1, False), (10, 1, 2, 1, True), (11, 1, 2, 1, False), (10, 1, 2, 2, False), (12, 2, 1, 1, False),
+    (13, 3, 1, 1, False), (15, 1, 1, 1, True), (16, 1, 2, 1, False), (16, 2, 1, 1, True)])
+def test_gradient_kernels_over_their_range(n, m, depth, bps, cplx):
+    """Every kind of lane: state counts with and without a padding half, in one block of the Z tile and in four, all
+    slot counts, real H and complex H with a bath frequency. Depth 2 and 3 put sqrt(n) and sqrt(n + 1) beyond 1 in.
+    Tolerances of the dense reference above: 1e-12 of the loss, 1e-9 of the largest entry (H, rho0), 1e-6 (lambda,
+    gamma: differences of 1e-4 relative, 1e-8 of the third derivative). Gradients that vanish (a single state) or happen
+    to be small are held to 1e-9 of what the norms of rho0 and O allow: `unit` bounds the loss, and times the sweep's
+    time over hbar its derivative by an energy, over lambda or gamma those by the bath's constants."""
+    h = complex_h(n, 70 + n) if cplx else ho.synthetic_hamiltonian(n, 70 + n)
+    lam, inv, omega, steps, dt_fs = 30.0, 60.0, (15.0 if cplx else 0.0), 6, 2.0
+    coupling = None
+    if bps == 2:  # bath i on sites i and i + 1, the last site with a single one
+        coupling = np.array([[i, (i + 1) % n] for i in range(n)], np.int32)
+        coupling[n - 1, 1] = -1
+    rng = np.random.default_rng(n * 100 + m)
+    rho0, obs = (rng.normal(size=(n, n)) + 1j * rng.normal(size=(n, n)) for _ in range(2))
+    w = hb.trapezoid_weights(steps, dt_fs)
+    pick = sorted({(0, 0), (n - 1, n - 1), (0, n - 1), (n - 1, 0), (n // 2, (n // 2 + 1) % n)})
+    J, gh, gl, gg, gr = tangent_gradients(n, h, lam, inv, m, depth, dt_fs, steps, rho0, obs, w, omega, coupling, pick,
+                                          pick[:3])
+    system = hb.System(h, [lam] * n, [inv] * n, [omega] * n, m, 300.0, depth, coupling=coupling)
+    with hb.Adjoint(system) as A:
+        out = A.gradient(rho0, obs, w, dt_fs * 1e-15, steps)
+    assert abs(out["loss"] - J) <= 1e-12 * max(1.0, abs(J))
+    unit = np.linalg.norm(rho0) * np.linalg.norm(obs) * np.sum(w)
+    scale = max(np.max(np.abs(out["h"])), unit * steps * dt_fs * 1e-15 * INVCM / 1.05457148e-34)
+    for (a, b), v in gh.items():
+        assert abs(out["h"][a, b] - v) <= 1e-9 * scale, (a, b, out["h"][a, b], v)
+    assert abs(out["lambda"] - gl) <= max(1e-6 * abs(gl), 1e-9 * unit / lam), (out["lambda"], gl)
+    assert abs(out["gamma"] - gg) <= max(1e-6 * abs(gg), 1e-9 * unit * inv), (out["gamma"], gg)
+    for (a, b), v in gr.items():
+        assert abs(out["rho0"][a, b] - v) <= 1e-9 * np.max(np.abs(out["rho0"])), (a, b)
+
+
+@pytest.mark.parametrize("n,depth,steps,group", [(7, 8, 14, 3), (9, 6, 8, 2)])
+def test_grouped_gradient_launches_with_a_remainder(n, depth, steps, group):
+    """The gradient contributions of `group` steps in one launch (by the 64 MB of their adjoint states) against one
+    launch per factor (any memory limit): bit for bit, where the group does not divide the segments of ceil(sqrt(steps))
+    steps."""
+    system = hb.System(ho.synthetic_hamiltonian(n, 9), [35.0] * n, [50.0] * n, [0.0] * n, 1, 300.0, depth)
+    state = int(hb.build_tables(system)["matrices"]) * (n * (n - 1) // 2 + (n + 1) // 2) * 32
+    segment = int(np.ceil(np.sqrt(steps)))
+    assert (64 << 20) // (4 * state) == group and segment > group and segment % group
+    rho0 = np.zeros((n, n), complex)
+    rho0[0, 0] = 1.0
+    obs = np.zeros((n, n), complex)
+    obs[1, 1], obs[0, 2] = 1.0, 0.5j
+    w = hb.trapezoid_weights(steps, 1.0)
+    with hb.Adjoint(system) as A:
+        grouped = A.gradient(rho0, obs, w, 1e-15, steps)
+        launches = A.kernel_launches()
+        A.set_memory_limit(1 << 40)
+        single = A.gradient(rho0, obs, w, 1e-15, steps)
+        assert A.recursive_slots() == 0 and A.kernel_launches() - launches > launches
+        A.set_memory_limit(0)
+        again = A.gradient(rho0, obs, w, 1e-15, steps)
+    for o in (single, again):
+        for k in ("loss", "h", "lambda", "gamma", "rho0"):
+            assert np.array_equal(o[k], grouped[k]), k
