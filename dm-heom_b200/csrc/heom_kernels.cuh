@@ -218,9 +218,10 @@ __device__ __forceinline__ void cmac(double2& acc, const double2 a, const double
 //
 // Pipeline: per warp two slots, each filled by two 1-D TMA bulk copies (tile,
 // record) that complete on the slot's mbarrier; the copies of ADO k+1 fly
-// while ADO k is computed.  Every wait is bounded and ends the same for all
-// lanes of the warp; on expiry the warp waits (bounded again) for the copies it
-// has in flight, sets *err and leaves as a whole.
+// while ADO k is computed.  Every wait is bounded.  The MMAs and shuffles are the
+// whole warp's work, so if the wait of a lane expires the warp leaves as a whole:
+// where it waits for the next ADO (two slots and more) once this one is done, else
+// at once.  It then waits, bounded again, for the copies in flight and sets *err.
 //
 // What bounds it: the L1 data pipe (8 states, two slots: 143 wavefronts of 194
 // cycles per ADO and SM; 88 of them shared memory) and the latency of 20 warps
@@ -347,25 +348,47 @@ __device__ __forceinline__ void mbar_expect(uint64_t* bar, unsigned bytes)
                  : "memory");
 }
 
-// tries of a bounded wait; an expression, so that a test can let the waits of chosen lanes run out
+// tries of a bounded wait (a second or so) and what a lane makes of one: a test may have chosen lanes overlook that
+// the phase is complete, with fewer tries
 #ifndef HEOM_WAIT_TRIES
 #define HEOM_WAIT_TRIES (1 << 24)
 #endif
+#ifndef HEOM_WAIT_SEEN
+#define HEOM_WAIT_SEEN(done, parity) (done)
+#endif
 
-// bounded wait for the phase `parity` of an mbarrier; false on expiry
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity, int tries)
+__device__ __forceinline__ bool mbar_try(uint64_t* bar, unsigned parity)
 {
-    const unsigned a = smem_addr(bar);
-    for (int it = 0; it < tries; ++it) {
-        unsigned done;
-        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-                     " selp.u32 %0, 1, 0, p;\n}\n"
-                     : "=r"(done)
-                     : "r"(a), "r"(parity)
-                     : "memory");
-        if (done) return true;
-    }
+    unsigned done;
+    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+                 " selp.u32 %0, 1, 0, p;\n}\n"
+                 : "=r"(done)
+                 : "r"(smem_addr(bar)), "r"(parity)
+                 : "memory");
+    return done != 0;
+}
+
+// bounded wait of a lane for the phase `parity` of an mbarrier; false on expiry
+__device__ __forceinline__ bool lane_wait(uint64_t* bar, unsigned parity)
+{
+    for (int it = 0; it < HEOM_WAIT_TRIES; ++it)
+        if (HEOM_WAIT_SEEN(mbar_try(bar, parity), parity)) return true;
     return false;
+}
+
+// the same of a whole warp, with one answer for every lane
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, unsigned parity)
+{
+    for (int it = 0; it < HEOM_WAIT_TRIES; ++it)
+        if (__all_sync(0xffffffffu, HEOM_WAIT_SEEN(mbar_try(bar, parity), parity))) return true;
+    return false;
+}
+
+// the time of a wait for copies that nothing is done with any more
+__device__ __forceinline__ void drain(uint64_t* bar, unsigned parity)
+{
+    for (int it = 0; it < HEOM_WAIT_TRIES && !mbar_try(bar, parity); ++it) {
+    }
 }
 
 // bytes of one pipeline slot and of a warp's shared area for the DMMA kernel:
@@ -582,16 +605,11 @@ __global__ void __launch_bounds__(kRowWarps * 32, row_blocks(HK, SLT, MI)) heom_
         }
     };
     unsigned it = 0; // ADOs done: slot it & 1, mbarrier parity (it >> 1) & 1
-    // whether the copies of the warp's k-th ADO have arrived: the same for every lane, since what follows is the whole
-    // warp's work (MMAs, shuffles) and a warp gives up as a whole
-    auto arrived = [&](unsigned k) {
-        return __all_sync(0xffffffffu, mbar_wait(bars + (k & 1), (k >> 1) & 1, HEOM_WAIT_TRIES)) != 0;
-    };
     bool failed = false;
     if (u < nodes) {
         if (lane == 0) issue(u, slot, bars);
         if (AHEAD) {
-            if (arrived(0)) load_k(slot, 0);
+            if (warp_wait(bars, 0)) load_k(slot, 0);
             else failed = true;
         }
     }
@@ -608,7 +626,7 @@ __global__ void __launch_bounds__(kRowWarps * 32, row_blocks(HK, SLT, MI)) heom_
             ni_ahead = u + 2 * stride < nodes ? __ldg(p.inst + u + 2 * stride) : ni;
         }
         if (!AHEAD) {
-            if (!arrived(it)) {
+            if (!warp_wait(bars + (it & 1), (it >> 1) & 1)) {
                 failed = true;
                 break;
             }
@@ -729,8 +747,8 @@ __global__ void __launch_bounds__(kRowWarps * 32, row_blocks(HK, SLT, MI)) heom_
         }
         // ---- the next ADO's K neighbours: in flight through the exchange, the stores and its commutator ----
         if (AHEAD && more) {
-            if (arrived(it + 1)) load_k(slot_n, 0);
-            else failed = true;
+            if (lane_wait(bars + ((it & 1) ^ 1), ((it + 1) >> 1) & 1)) load_k(slot_n, 0);
+            else failed = true; // (the warp leaves as a whole, after this ADO)
         }
         // ---- the handed-over sector's terms to its owner ----
         const double2 hf = shfl2(gf, giver), hs = shfl2(gs, giver);
@@ -763,6 +781,7 @@ __global__ void __launch_bounds__(kRowWarps * 32, row_blocks(HK, SLT, MI)) heom_
             }
         }
         __syncwarp();
+        if (AHEAD) failed = __any_sync(0xffffffffu, failed);
         unsigned char* const sw = slot;
         slot = slot_n;
         slot_n = sw;
@@ -780,8 +799,8 @@ __global__ void __launch_bounds__(kRowWarps * 32, row_blocks(HK, SLT, MI)) heom_
     // a warp whose wait expired flags the launch as failed; before it leaves, the copies that no wait has seen arrive
     // (ADO it's, and the next one's where it was issued before that wait) get their time to land
     if (failed) {
-        mbar_wait(bars + (it & 1), (it >> 1) & 1, 1 << 24);
-        if (!AHEAD && u + stride < nodes) mbar_wait(bars + ((it & 1) ^ 1), ((it + 1) >> 1) & 1, 1 << 24);
+        drain(bars + (it & 1), (it >> 1) & 1);
+        if (!AHEAD && u + stride < nodes) drain(bars + ((it & 1) ^ 1), ((it + 1) >> 1) & 1);
         if (lane == 0) *static_cast<volatile int*>(dp.err) = 1;
     }
 }

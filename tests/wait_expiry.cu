@@ -1,21 +1,21 @@
 // A pipeline wait of the N <= 8 stage kernel that runs out (compiled and run by tests/test_gpu_wait.py).  The copies
-// themselves arrive; chosen lanes are given no tries to see it.  With no H, bath term or same term the stage is
+// themselves arrive; chosen lanes overlook it.  With no H, bath term or same term the stage is
 // out = in, so that what a warp wrote before it gave up can be told from what it did not.  Prints "bad ..." for any
 // violation, then "ok" or "FAILED".
 #include <cstdint>
 #include <cstdio>
 #include <vector>
 
-// mode 0: every wait has its tries; 1: lane 5 has none; 2: no lane has any; 3: lane 5 has none in its third wait
+// mode 0: every lane sees its copies arrive; 1: lane 5 never does; 2: no lane does; 3: lane 5 does not in its third
+// wait (the first of the warp's two mbarriers, its second phase)
 __constant__ int c_mode;
-__device__ int g_waits[1 << 16];
-__device__ inline int wait_tries()
+__device__ inline bool wait_seen(bool done, unsigned parity)
 {
-    const int w = g_waits[blockIdx.x * blockDim.x + threadIdx.x]++;
     const bool five = threadIdx.x % 32 == 5;
-    return c_mode == 2 || (c_mode == 1 && five) || (c_mode == 3 && five && w == 2) ? 0 : 1 << 24;
+    return done && !(c_mode == 2 || (c_mode == 1 && five) || (c_mode == 3 && five && parity == 1));
 }
-#define HEOM_WAIT_TRIES wait_tries()
+#define HEOM_WAIT_SEEN(done, parity) wait_seen(done, parity)
+#define HEOM_WAIT_TRIES (1 << 14)
 #include "heom_kernels.cuh"
 #include "row_tables.inc"
 
@@ -83,9 +83,7 @@ void run(const char* name, void (*kernel)(const heomk::DmmaParams))
     const int warps = blocks * heomk::kRowWarps;
     for (int mode : {0, 1, 2, 3, 0}) {
         if (bad) return;
-        const std::vector<int> none(1 << 16, 0);
         TRY(cudaMemcpyToSymbol(c_mode, &mode, sizeof mode));
-        TRY(cudaMemcpyToSymbol(g_waits, none.data(), none.size() * sizeof(int)));
         TRY(cudaMemcpy(dp.p.out, mark.data(), mark.size() * 16, cudaMemcpyHostToDevice));
         *static_cast<volatile int*>(err) = 0;
         kernel<<<blocks, heomk::kRowWarps * 32, smem>>>(dp);
