@@ -253,11 +253,12 @@ struct RowTab {
 };
 
 // lane tables of the lockstep kernel: the operand sectors of every lane and
-// which half holds the row element
+// which half holds the row element.  A lane outside N x N has those of a lane
+// of its quarter warp that is inside and not on the diagonal (where there is one).
 struct LaneTab {
     signed char e1[32], e2[32]; // sector of lane p: element indices (row-major)
     signed char ord[32];        // the sectors in the order in which the warps take them
-    signed char fs[32][2];      // operand sector of k-slice s (-1: zero padding)
+    signed char fs[32][2];      // operand sector of k-slice s
     signed char ha[32][2];      // half of that sector holding A = w(r, 2t+s)
 };
 

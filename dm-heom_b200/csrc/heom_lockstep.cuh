@@ -141,9 +141,10 @@ __global__ void __launch_bounds__(kLockWarps * 32, 2) heom_lockstep_stage(const 
     const int r = lane >> 2, t = lane & 3;
     // Phase A offsets (double2, from a tile buffer) of this lane's operands for the warp's first
     // instance; its instance warp + 8 j adds 16 j, since the column swizzle k ^ (p & 3) changes
-    // bits 0-1 of k only. An operand outside the N x N block reads an arbitrary finite tile value
-    // (sector 0): its partner fragment of H is zero, so it adds only zeros, to rows and columns
-    // that are not read.
+    // bits 0-1 of k only. A lane outside the N x N block reads what a lane of its quarter warp inside it
+    // reads (LaneTab), which costs no wavefront: its partner fragment of H is zero, so it adds only zeros
+    // as long as the value is finite, and it is one of the same instance, so that a realisation that has
+    // diverged stays by itself.
     // Shared tiles store half h of instance column k at position h ^ ((k >> 2) & 1): a warp's
     // 16-byte accesses to one half of 32 columns then cover all eight 16-byte bank groups.
     const int hw = (warp >> 2) & 1; // (k >> 2) & 1 of the warp's phase A instances
@@ -151,13 +152,13 @@ __global__ void __launch_bounds__(kLockWarps * 32, 2) heom_lockstep_stage(const 
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
         const int fs = s == 0 ? fs0 : fs1, ha = s == 0 ? ha0 : ha1;
-        const int row = fs >= 0 ? (fs * 32 + (warp ^ (fs & 3))) * 2 : 0;
-        oa[s] = fs >= 0 ? row + (ha ^ hw) : 0;
-        ob[s] = fs >= 0 ? (r == 2 * t + s ? row + (ha ^ hw) : row + (ha ^ 1 ^ hw)) : 0; // diagonal: its own transpose
+        const int row = (fs * 32 + (warp ^ (fs & 3))) * 2;
+        oa[s] = row + (ha ^ hw);
+        ob[s] = row + (r < N && r == 2 * t + s ? ha ^ hw : ha ^ 1 ^ hw); // diagonal: its own transpose
     }
     // the MMA result is the lane's own row elements (r, 2t), (r, 2t+1): the commutator of element (r, 2t+s) goes
     // where the A operand of slice s was read (elements outside the N x N block: a row that is not read)
-    const int oc0 = fs0 >= 0 ? oa[0] : P * 64, oc1 = fs1 >= 0 ? oa[1] : P * 64;
+    const int oc0 = r < N && 2 * t < N ? oa[0] : P * 64, oc1 = r < N && 2 * t + 1 < N ? oa[1] : P * 64;
     const int hk = (lane >> 2) & 1; // phase B: position of half 0 of this lane's instance
     // the slot of site (lane / SLT) that lane of the table warp resolves
     const int tsite = lane / SLT, tq = lane - tsite * SLT;

@@ -1011,19 +1011,18 @@ int build_pair_tables(heom_handle* h, bool lockstep = false)
             const int r = l >> 2, t = l & 3;
             for (int s = 0; s < 2; ++s) {
                 const int k = 2 * t + s;
+                const bool in = r < N && k < N;
+                // outside N x N: element (2q + 1, 0) of the lane's quarter q, or (2q, 1), else the quarter's last state
+                const int r2 = in ? r : std::min(2 * (r / 2) + (s ? 0 : 1), N - 1), k2 = in ? k : std::min(s, N - 1);
                 lt.fs[l][s] = -1;
-                lt.ha[l][s] = 0;
-                if (r < N && k < N) {
-                    const int e = r * N + k;
-                    for (int p = 0; p < P && lt.fs[l][s] < 0; ++p)
-                        for (int hf = 0; hf < 2 && lt.fs[l][s] < 0; ++hf)
-                            if (h->pair_tab[2 * p + hf] == e) {
-                                lt.fs[l][s] = (signed char)p;
-                                lt.ha[l][s] = (signed char)hf;
-                            }
-                    if (lt.fs[l][s] < 0) return fail(HEOM_E_UNSUPPORTED, "pair table misses element %d", e);
-                }
-                h->row_tab.pos[l][s] = lt.fs[l][s];
+                for (int p = 0; p < P && lt.fs[l][s] < 0; ++p)
+                    for (int hf = 0; hf < 2 && lt.fs[l][s] < 0; ++hf)
+                        if (h->pair_tab[2 * p + hf] == r2 * N + k2) {
+                            lt.fs[l][s] = (signed char)p;
+                            lt.ha[l][s] = (signed char)hf;
+                        }
+                if (lt.fs[l][s] < 0) return fail(HEOM_E_UNSUPPORTED, "pair table misses element %d", r2 * N + k2);
+                h->row_tab.pos[l][s] = in ? lt.fs[l][s] : (signed char)-1;
             }
         }
         // the diagonal sectors, whose bath terms are half of the others', all go to the first warp of the lockstep

@@ -178,3 +178,24 @@ def test_ensemble_splits_a_class_into_lockstep_and_mixed_depths():
         tops = E.propagate(DT, 30, 10)
     for k in (0, 9, 10, 12):
         assert np.array_equal(tops[k], alone(probs[k], 30, 10)), f"instance {k}"
+
+
+@pytest.mark.parametrize("n,m,depth,complex_h", [(7, 1, 2, False), (5, 2, 2, True), (8, 1, 2, False)])
+def test_diverged_realisation_of_a_lockstep_class_stays_by_itself(n, m, depth, complex_h):
+    """A realisation that is not finite any more leaves the others of its block of 32 as they are without it."""
+    count, lost = 40, (0, 33)
+    probs = disorder_problems(count, n, [depth], m, seed=7, complex_h=complex_h)
+    with hb.Ensemble([hb.Heom.tables_of(p) for p in probs]) as E:
+        assert E.classes() == 1
+        got = []
+        for bad in (False, True):
+            E.clear()
+            for k in range(count):
+                E.set_top(k, np.full(n * n * 2, np.nan) if bad and k in lost else top0(n))
+            E.rk4_steps(DT, 2)
+            got.append([E.get_top(k) for k in range(count)])
+    for k in range(count):
+        if k in lost:
+            assert not np.any(np.isfinite(got[1][k]))
+        else:
+            assert np.array_equal(got[1][k], got[0][k]), k
