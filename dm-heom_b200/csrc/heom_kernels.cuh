@@ -131,12 +131,14 @@ __host__ __device__ constexpr int tile_pos(int n, int i, int k) { return i * til
 constexpr int kXchStride = 17;
 constexpr int kXchBytes = 16 * kXchStride * 16;
 
-// shared look-up tables of both stage kernels: khat 3*W double2, (sqrt(n),
-// sqrt(n+1)) LS+1 double2, chat W doubles, pos W int16 (the last read by the
-// team kernel only)
+// shared look-up tables of the stage kernels: khat 3*W double2, (sqrt(n),
+// sqrt(n+1)) LS+1 double2, chat W doubles; padded to 128 bytes, since the tiles
+// of the lockstep kernel follow: off a 32-byte boundary they cost 4 to 6 % (256
+// instances of 7 states, depth 6: 217 -> 226 us a stage; 128 of 8, depth 5: 98.7
+// -> 105.3; on a 128-byte boundary 219.8 and 97.2)
 __host__ __device__ inline int dmma_lut_bytes(int W, int LS)
 {
-    return ((3 * W * 16 + (LS + 1) * 16 + W * 8 + W * 2) + 15) & ~15;
+    return ((3 * W * 16 + (LS + 1) * 16 + W * 8) + 127) & ~127;
 }
 
 // dynamic shared memory carve-up (bytes); everything 16-B aligned
@@ -223,22 +225,25 @@ __device__ __forceinline__ void cmac(double2& acc, const double2 a, const double
 // where it waits for the next ADO (two slots and more) once this one is done, else
 // at once.  It then waits, bounded again, for the copies in flight and sets *err.
 //
-// What bounds it: the L1 data pipe (8 states, two slots: 143 wavefronts of 194
-// cycles per ADO and SM; 88 of them shared memory) and the latency of 20 warps
-// per SM.  Measured against a lane per sector, which looked up both sites'
+// What bounds it: the L1 data pipe (8 states, two slots, 245,157 ADOs: 135
+// wavefronts in 201 cycles per ADO and SM, 75 of them shared memory) and the
+// latency of 20 warps per SM; on 735,471 ADOs of a state beyond L2 DRAM is the
+// nearer limit (1.83 x the algorithmic bytes).  Measured against a lane per sector, which looked up both sites'
 // slots for two elements (us per stage, one B200): 8 states, two slots, 735,471
 // ADOs 791 -> 547, 74,613 ADOs 76.0 -> 51.8; one slot, 24,310 ADOs 21.5 -> 14.9,
 // 319,770 ADOs 235 -> 217; 7 states, one slot, 6435 ADOs 9.75 -> 6.6; 330 ADOs
-// 4.6 -> 3.1 (mostly the dependent launch).  503 -> 347 instructions and 204 ->
-// 143 wavefronts per ADO; 47 of the 61 fewer are shared memory's, the rest a
-// store that is linear in the lanes (22 -> 8) and owned sectors side by side.
+// 4.6 -> 3.1 (mostly the dependent launch).  503 -> 352 instructions and 204 ->
+// 135 wavefronts per ADO; most of the fewer are shared memory's (130 -> 75), the
+// rest a store that is linear in the lanes (22 -> 8) and owned sectors side by side.
 // A lane table read from the parameter bank has to be held (opaque): reloaded
 // under register pressure it cost 180 instructions per ADO and half the speed.
 // Two slots: the K neighbours are read one ADO ahead and the coefficients come
 // from shared memory (in registers they spill: 1137 us); one slot: the other
 // way round.  Two slots: reading the real parts of the same term's factors alone
 // and the own sector's halves in a staggered order took 13 wavefronts more:
-// 74,613 ADOs 50.1, 735,471 ADOs 540.
+// 74,613 ADOs 50.1, 735,471 ADOs 540.  The votes by which a warp leaves as a whole
+// cost 0.4 % (74,613 ADOs 50.35), 6435 ADOs of 7 states 1.5 % (6.31 -> 6.40); with
+// the vote in every lane's way to its loads 74,613 ADOs took 51.0.
 // ---------------------------------------------------------------------------
 
 // which of its two sectors lane (r, t) owns: 0 = {r, 2t}, 1 = {r, 2t+1}
@@ -287,14 +292,8 @@ __device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b)
                  : "d"(a), "d"(b));
 }
 
+// 32 bytes through the coherent path: a stage runs as a dependent of the kernel that writes what it reads
 __device__ __forceinline__ void ld256(const double2* src, double2& a, double2& b)
-{
-    asm volatile("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];\n"
-                 : "=d"(a.x), "=d"(a.y), "=d"(b.x), "=d"(b.y)
-                 : "l"(src));
-}
-
-__device__ __forceinline__ void ld256_cg(const double2* src, double2& a, double2& b)
 {
     asm volatile("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];\n"
                  : "=d"(a.x), "=d"(a.y), "=d"(b.x), "=d"(b.y)
@@ -451,7 +450,12 @@ constexpr int row_blocks(int hk, int slt, bool mi) { return hk == H_REAL_SYM && 
 // with conj(khat) sqrt(n+1), the minus neighbour with -/+ i chat sqrt(n).
 // "K" is the neighbour with the complex coefficient (minus for L, plus for
 // L^H), "C" the one with the imaginary coefficient.
-// GEN: every write mode; otherwise out = in + beta L only (the product form).
+// GEN: every write mode; otherwise out = in + beta L only (the product form), whose
+// epilogue tests no mode and holds no pointer for one.  us per stage of the product
+// form through the first / the second: 8 states, two slots, 74,613 ADOs 52.2 / 50.7,
+// 735,471 ADOs 552 / 545; one slot, 24,310 ADOs 15.9 / 15.2; 7 states, one slot, 6435
+// ADOs 6.60 / 6.24; 4 states, three slots, 18,564 ADOs 18.5 / 17.4; 6 states, one
+// slot, 8008 ADOs 7.22 / 7.18.
 template <int N, int HK, int SLT, bool MI, bool ADJ, bool GEN>
 __global__ void __launch_bounds__(kRowWarps * 32, row_blocks(HK, SLT, MI)) heom_dmma_stage(const __grid_constant__ DmmaParams dp)
 {
@@ -767,7 +771,7 @@ __global__ void __launch_bounds__(kRowWarps * 32, row_blocks(HK, SLT, MI)) heom_
             }
             double2 o1 = xf, o2 = xs;
             if (GEN) {
-                if (p.y) ld256_cg(p.y + off, o1, o2);
+                if (p.y) ld256(p.y + off, o1, o2);
                 if (!p.use_x) o1 = o2 = make_double2(0.0, 0.0);
             }
             cmac(o1, p.beta, L1);
@@ -775,7 +779,7 @@ __global__ void __launch_bounds__(kRowWarps * 32, row_blocks(HK, SLT, MI)) heom_
             st256_cs(p.out + off, o1, o2);
             if (GEN && p.use_acc) {
                 double2 a1 = xf, a2 = xs;
-                if (!p.acc_init) ld256_cg(p.acc + off, a1, a2);
+                if (!p.acc_init) ld256(p.acc + off, a1, a2);
                 cmac(a1, p.acc_beta, L1);
                 cmac(a2, p.acc_beta, L2);
                 st256(p.acc + off, a1, a2);
@@ -834,9 +838,11 @@ __global__ void __launch_bounds__(kRowWarps * 32, row_blocks(HK, SLT, MI)) heom_
 // Instruction issue and the L1 data pipe bound it.  us per stage, one B200: 256
 // instances of 7 states, depth 6: 245.3 -> 244.3 with the list and absent
 // neighbours skipped (the terms of both sides now add up as heom_dmma_stage's
-// do), -> 225.3 without an exchange of the commutator through shared memory;
-// 40 at depth 4: 18.8 -> 16.3 -> 14.7; 64 of 6 states, two slots, depth 4: 69.5
-// -> 68.7 -> 62.9.
+// do), -> 224.5 without an exchange of the commutator through shared memory, ->
+// 219.8 with lanes outside the tile reading what one inside reads and sectors in an
+// order searched for the reads that are made; 40 at depth 4: 18.8 -> 16.3 -> 14.4 ->
+// 14.0; 256 of 6 states, depth 6: 107 -> 101 by the last step; 64 of 6 states, two
+// slots, depth 4: 69.5 -> 68.7 -> 62.9 -> 57.4.
 // ---------------------------------------------------------------------------
 
 // ---------------------------------------------------------------------------
@@ -862,7 +868,7 @@ __global__ void __launch_bounds__(kRowWarps * 32, row_blocks(HK, SLT, MI)) heom_
 // that no second barrier is needed.
 //
 // What bounds it: 18 to 20 warps per SM (96 registers) with the L1 data pipe
-// 69 % busy (12 states, two slots: 512 wavefronts of 747 cycles per ADO and SM,
+// 63 % busy (12 states, two slots: 514 wavefronts in 815 cycles per ADO and SM,
 // 373 of them shared memory) and the FP64 tensor pipe a quarter.  Measured
 // against a thread per sector with two barriers per ADO (us per stage, one
 // B200): 12 states, two slots, 20,475 ADOs 74.5 -> 55.5 (24 warps of 80
@@ -1072,7 +1078,7 @@ __global__ void __launch_bounds__(team_threads(N), team_blocks(N, HK, SLT))
         // what the stage adds to: y takes the place of the own values, in flight through the bath terms (a launch with
         // y never starts acc from the own values)
         double2 x1 = xf, x2 = xs;
-        if (p.y && owner) ld256_cg(p.y + (int64_t)u * (2 * P) + 2 * pso, x1, x2);
+        if (p.y && owner) ld256(p.y + (int64_t)u * (2 * P) + 2 * pso, x1, x2);
 #pragma unroll
         for (int q0 = 0; q0 < SLT; q0 += QB) {
             if (q0 > 0) {
@@ -1153,7 +1159,7 @@ __global__ void __launch_bounds__(team_threads(N), team_blocks(N, HK, SLT))
             st256_cs(p.out + off, r1, r2);
             if (p.use_acc) {
                 double2 a1 = x1, a2 = x2;
-                if (!p.acc_init) ld256_cg(p.acc + off, a1, a2);
+                if (!p.acc_init) ld256(p.acc + off, a1, a2);
                 cmac(a1, p.acc_beta, L1);
                 cmac(a2, p.acc_beta, L2);
                 st256(p.acc + off, a1, a2);
@@ -1294,7 +1300,7 @@ __global__ void heom_write_top(double2* __restrict__ y, const double2* __restric
 // stage kernels in turn, so that the look-ups of a slot serve four elements, and
 // the derivative tables lie in shared memory.  Latency bounds it, so that two
 // blocks on an SM count for more than the 32 bytes that 128 registers spill, and
-// a warp's sums lie where its tiles were (16 states: 90 KB a block).  Whole
+// a warp's sums lie where its tiles were (16 states: 86 KB a block).  Whole
 // gradient calls, one B200, with one block of 158 registers -> with two: 4
 // instances of 9 states, 715 ADOs each, 40 steps 7220 -> 6910 us; 12 states, two
 // slots, 20,475 ADOs, 8 steps 10,840 -> 9150; 16 states, 4845 ADOs, 20 steps
@@ -1420,8 +1426,8 @@ __global__ void __launch_bounds__(kCtaWarps * 32, 2) heom_adjoint_grad(const __g
                 const GradLane q = lanes[l];
                 if (q.pso < 0) continue;
                 double2 a1, a2, w1, w2;
-                ld256_cg(a_in + (u * P + q.pso) * 2, a1, a2);
-                ld256_cg(w_in + (u * P + q.pso) * 2, w1, w2);
+                ld256(a_in + (u * P + q.pso) * 2, a1, a2);
+                ld256(w_in + (u * P + q.pso) * 2, w1, w2);
                 At[q.q1] = a1;
                 At[q.q2] = a2;
                 Wt[q.q1] = w1;
@@ -1649,8 +1655,8 @@ __global__ void __launch_bounds__(kCtaWarps * 32, 2) heom_row_grad(const __grid_
             double2 xo[2], xg[2]; // minus neighbour
             const int64_t o = (int64_t)u * (2 * P);
             if (owner) {
-                ld256_cg(a_in + o + 2 * pso, a1, a2);
-                ld256_cg(w_in + o + 2 * pso, w1, w2);
+                ld256(a_in + o + 2 * pso, a1, a2);
+                ld256(w_in + o + 2 * pso, w1, w2);
             }
             const double dps = g.dpss[u];
             int2 cm[SLT];
