@@ -227,9 +227,10 @@ __device__ __forceinline__ void cmac(double2& acc, const double2 a, const double
 //
 // What bounds it: the L1 data pipe (8 states, two slots, 245,157 ADOs: 135
 // wavefronts in 201 cycles per ADO and SM, 75 of them shared memory) and the
-// latency of 20 warps per SM; on 735,471 ADOs of a state beyond L2 DRAM is the
-// nearer limit (1.83 x the algorithmic bytes).  Measured against a lane per sector, which looked up both sites'
-// slots for two elements (us per stage, one B200): 8 states, two slots, 735,471
+// latency of 20 warps per SM; on 735,471 ADOs, a state beyond L2, DRAM is the
+// nearer limit (1.84 x the algorithmic bytes).  Measured against a lane per
+// sector, which looked up both sites' slots for two elements (us per stage, one
+// B200): 8 states, two slots, 735,471
 // ADOs 791 -> 547, 74,613 ADOs 76.0 -> 51.8; one slot, 24,310 ADOs 21.5 -> 14.9,
 // 319,770 ADOs 235 -> 217; 7 states, one slot, 6435 ADOs 9.75 -> 6.6; 330 ADOs
 // 4.6 -> 3.1 (mostly the dependent launch).  503 -> 352 instructions and 204 ->
@@ -872,9 +873,12 @@ __global__ void __launch_bounds__(kRowWarps * 32, row_blocks(HK, SLT, MI)) heom_
 // 373 of them shared memory) and the FP64 tensor pipe a quarter.  Measured
 // against a thread per sector with two barriers per ADO (us per stage, one
 // B200): 12 states, two slots, 20,475 ADOs 74.5 -> 55.5 (24 warps of 80
-// registers: 66) -> 53.4 with y read before the barrier, one slot, 18,564 ADOs 51.9 -> 43.1; 10 states, two slots,
-// 10,626 ADOs 29.4 -> 24.4; 9 states, one slot, 5005 ADOs 13.9 -> 11.8; 11
-// states (three warps instead of two), one slot, 12,376 ADOs 29.3 -> 28.6.
+// registers: 66) -> 53.4 with y read before the barrier, one slot, 18,564 ADOs
+// 51.9 -> 43.1; 10 states, two slots, 10,626 ADOs 29.4 -> 24.4; 9 states, one
+// slot, 5005 ADOs 13.9 -> 11.8; 11 states (three warps instead of two), one slot,
+// 12,376 ADOs 29.3 -> 28.6; 16 states, two slots, 6545 ADOs 34.0 -> 27.3, one
+// slot, 969 ADOs 8.21 -> 7.18, but 20,349 ADOs 75.2 -> 76.1 (with 106 registers
+// and 16 warps 78.2).
 // ---------------------------------------------------------------------------
 
 // position of the sector owned by thread (r, t): threads of odd rows own
